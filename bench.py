@@ -320,7 +320,7 @@ def time_form(args, precision, tp, ic, local, pg, profile_names):
     return ms, launches, prof, sim
 
 
-PROFILE_NAMES = ("k_hydro_stage_fp32", "k_faces_fp64", "k_hydro_update_fp64", "k_q_from_u", "k_dt_reduce",
+PROFILE_NAMES = ("k_hydro_stage_fp32", "k_faces", "k_hydro_update_fp64", "k_q_from_u", "k_dt_reduce",
                  "k_dt_finalize", "k_dt_reset", "k_time_advance", "graph_rad_sweep", "graph_colden_sweep",
                  "k_rad_shell", "k_colden_shell", "k_thermo", "k_rad_heating", "k_rad_update", "k_rad_wind",
                  "k_rad_no_star")
@@ -424,7 +424,7 @@ def run_batch(args, world, rank, local, pg):
     # roofline of the HBM-bound kernel with the largest share among those with a
     # stated algorithmic byte count per cell (FP64 form)
     # (the FP32 form's batch hydro pass: read U, write U1 and Q, then U1 back to U)
-    per_cell = {"k_hydro_update_fp64": 280.0, "k_faces_fp64": 112.0, "k_q_from_u": 112.0,
+    per_cell = {"k_hydro_update_fp64": 280.0, "k_faces": 112.0, "k_q_from_u": 112.0,
                 "k_hydro_stage_fp32": 280.0}
     roofline = None
     cand = [(v["ms"], k) for k, v in prof.items() if k in per_cell]
@@ -751,10 +751,10 @@ def run_ours(args, world, rank, local, pg):
         # FP64 state, reading U (7 x 8 B) and writing the new U and its Q (2 x 7 x 8 B)
         alg_per_launch = 168.0 * N
     else:
-        kname = "k_faces_fp64"
-        # FP64 plain form, per face-flux launch (one per dimension, 2 stages):
-        # reads the 7 primitive fields (8 B each) and writes 7 flux fields
-        alg_per_launch = (7 * 8 + 7 * 8) * N
+        kname = "k_faces"
+        # FP64 plain form, per face-flux launch (all dimensions): reads the 7
+        # primitive fields (8 B each) and writes 7 flux fields per dimension
+        alg_per_launch = (7 * 8 + 7 * 8 * int(ic.nd)) * N
     tot_ms, count = prof.get(kname, (0.0, 0))
     avg_ms = tot_ms / count if count else float("nan")
     achieved = alg_per_launch / (avg_ms / 1e3) / 1e9 if count else None

@@ -377,7 +377,25 @@ void comp_pre(trg_ctx* c, int comp) {
 
 void hydro_fluxes(trg_ctx* c) {
 	halo_exchange(c, c->S.Q, false);
-	for (int d = 0; d < c->P.nd; ++d) LAUNCH(KF(k_faces_fp64), c->S.nfaces[d], 128, c->P, c->S, d);
+	const Params& P = c->P;
+	if (P.batch) {
+		for (int d = 0; d < P.nd; ++d) LAUNCH(KF(k_faces_batch_fp64), c->S.nfaces[d], 128, P, c->S, d);
+		return;
+	}
+	// Faces per thread along y and z: long chunks save loads and slopes (each
+	// starts with three cells and one slope of its own), short ones keep the
+	// GPU full: about 6 blocks of 128 threads per SM.
+	const long long threads = 148LL * 6 * 128;
+	FaceGrid G;
+	G.chunk = (int)std::min<long long>(32, std::max<long long>(1, P.N * (P.nd - 1) / threads));
+	const long long xw = (long long)P.ny * P.nz * ((P.nx + 29) / 29);
+	G.bx = grid_for(xw, 4);
+	G.by = P.nd > 1 ? grid_for((long long)P.nx * P.nz * ((P.ny + G.chunk) / G.chunk), 128) : 0;
+	const long long bz = P.nd > 2 ? grid_for((long long)P.nx * P.ny * ((P.nz + G.chunk) / G.chunk), 128) : 0;
+	const long long n = (G.bx + G.by + bz) * 128;
+	if (P.nd == 3) LAUNCH(KF(k_faces3_fp64), n, 128, P, c->S, G);
+	else if (P.nd == 2) LAUNCH(KF(k_faces2_fp64), n, 128, P, c->S, G);
+	else LAUNCH(KF(k_faces1_fp64), n, 128, P, c->S, G);
 }
 
 // Single grids: the shells read their cells' own inputs in sweep order

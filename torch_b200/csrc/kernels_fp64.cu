@@ -32,306 +32,7 @@
 namespace trg {
 namespace TRG_KNS {
 
-// ------------------------------------------------------------------ limiters
-__device__ __forceinline__ double minmod(double a, double b) { return (a * b > 0) ? (fabs(a) < fabs(b) ? a : b) : 0; }
-__device__ __forceinline__ double maxmod(double a, double b) { return (a * b > 0) ? (fabs(a) > fabs(b) ? a : b) : 0; }
-
-// SlopeLimiter::calculate variants, SlopeLimiter.cpp:5-54.
-__device__ __forceinline__ double limiter(int kind, double a, double b) {
-	switch (kind) {
-	case 0: return minmod((a + b) / 2.0, minmod(2.0 * a, 2.0 * b));
-	case 1: return maxmod(minmod(b, 2.0 * a), minmod(2.0 * b, a));
-	case 2: return minmod(a, b);
-	case 3: return maxmod(a, b);
-	case 4: {
-		if (b == 0) return 0;
-		double r = fabs(a / b);
-		return (a + b * r) / (1.0 + r);
-	}
-	case 5: return (a * b <= 1.0e-30) ? 0 : 1.5 * b * (a * a + a * b) / (a * a + a * b + b * b);
-	default: return a * b <= 1.0e-30 ? 0 : a * b * (a + b) / (a * a + b * b);
-	}
-}
-
-// ----------------------------------------------------------- Riemann solvers
-// characteristicWaveSpeeds (Einfeldt), Riemann.cpp:27-42.
-__device__ __forceinline__ void wave_speeds(double a_l2, double a_r2, const double* Ql, const double* Qr, int dim,
-                                            double& Sl, double& Sr) {
-	double sqrtrho_l = sqrt(Ql[DEN]);
-	double sqrtrho_r = sqrt(Qr[DEN]);
-	double u_tilde = (sqrtrho_l * Ql[VEL + dim] + sqrtrho_r * Qr[VEL + dim]) / (sqrtrho_l + sqrtrho_r);
-	double nu2 = 0.5 * sqrtrho_r * sqrtrho_l / ((sqrtrho_l + sqrtrho_r) * (sqrtrho_l + sqrtrho_r));
-	double dsqrd = (sqrtrho_l * a_l2 + sqrtrho_r * a_r2) / (sqrtrho_l + sqrtrho_r);
-	dsqrd += nu2 * (Qr[VEL + dim] - Ql[VEL + dim]) * (Qr[VEL + dim] - Ql[VEL + dim]);
-	double d = sqrt(dsqrd);
-	Sl = u_tilde - d;
-	Sr = u_tilde + d;
-}
-
-// HartenLaxLeerContactSolver::solve, Riemann.cpp:52-104.
-__device__ void hllc(double* F, const double* Ql, const double* Qr, double a_l2, double a_r2, double gamma, int nd, int dim) {
-	double S_l, S_r;
-	wave_speeds(a_l2, a_r2, Ql, Qr, dim, S_l, S_r);
-	if (S_l >= 0) {
-		FfromQ(F, Ql, gamma, nd, dim);
-	} else if (S_r <= 0) {
-		FfromQ(F, Qr, gamma, nd, dim);
-	} else {
-		double S_c = Qr[PRE] - Ql[PRE];
-		S_c += Ql[DEN] * Ql[VEL + dim] * (S_l - Ql[VEL + dim]);
-		S_c -= Qr[DEN] * Qr[VEL + dim] * (S_r - Qr[VEL + dim]);
-		S_c /= (Ql[DEN] * (S_l - Ql[VEL + dim]) - Qr[DEN] * (S_r - Qr[VEL + dim]));
-		const double* Qlr = (S_c >= 0) ? Ql : Qr;
-		double S_lr = (S_c >= 0) ? S_l : S_r;
-		double U_lr[7] = {0, 0, 0, 0, 0, 0, 0}, F_lr[7] = {0, 0, 0, 0, 0, 0, 0}, U_c[7] = {0, 0, 0, 0, 0, 0, 0};
-		UfromQ(U_lr, Qlr, gamma, nd);
-		FfromQ(F_lr, Qlr, gamma, nd, dim);
-		double A_lr = Qlr[DEN] * (S_lr - Qlr[VEL + dim]) / (S_lr - S_c);
-		U_c[DEN] = A_lr;
-		#pragma unroll
-		for (int id = 0; id < 3; ++id) if (id < nd) U_c[VEL + id] = A_lr * Qlr[VEL + id];
-		U_c[VEL + dim] = A_lr * S_c;
-		U_c[PRE] = A_lr * ((U_lr[PRE] / Qlr[DEN]) +
-		                   (S_c - Qlr[VEL + dim]) * (S_c + Qlr[PRE] / (Qlr[DEN] * (S_lr - Qlr[VEL + dim]))));
-		U_c[HII] = A_lr * Qlr[HII];
-		U_c[ADV] = A_lr * Qlr[ADV];
-		for (int i = 0; i < NU; ++i) F[i] = F_lr[i] + S_lr * (U_c[i] - U_lr[i]);
-		if (nd < 3) F[VEL + 2] = 0;
-		if (nd < 2) F[VEL + 1] = 0;
-	}
-}
-
-// HartenLaxLeerSolver::solve, Riemann.cpp:108-140.
-__device__ void hll(double* F, const double* Ql, const double* Qr, double a_l2, double a_r2, double gamma, int nd, int dim) {
-	double S_l, S_r;
-	wave_speeds(a_l2, a_r2, Ql, Qr, dim, S_l, S_r);
-	if (S_r <= 0) {
-		FfromQ(F, Qr, gamma, nd, dim);
-	} else if (S_l >= 0) {
-		FfromQ(F, Ql, gamma, nd, dim);
-	} else {
-		double U_l[7] = {0, 0, 0, 0, 0, 0, 0}, U_r[7] = {0, 0, 0, 0, 0, 0, 0};
-		double F_l[7] = {0, 0, 0, 0, 0, 0, 0}, F_r[7] = {0, 0, 0, 0, 0, 0, 0};
-		UfromQ(U_l, Ql, gamma, nd);
-		UfromQ(U_r, Qr, gamma, nd);
-		FfromQ(F_l, Ql, gamma, nd, dim);
-		FfromQ(F_r, Qr, gamma, nd, dim);
-		for (int i = 0; i < NU; ++i)
-			F[i] = (S_r * F_l[i] - S_l * F_r[i] + S_l * S_r * (U_r[i] - U_l[i])) / (S_r - S_l);
-	}
-}
-
-// 3-vector helpers with the reduction order of the reference's vendored
-// Eigen 3.2.1 (x + (y + z) for dot/norm; v /= s multiplies by 1/s; matrix
-// coefficients accumulate (a + b) + c).
-__device__ __forceinline__ void cross3(const double* a, const double* b, double* r) {
-	r[0] = a[1] * b[2] - a[2] * b[1];
-	r[1] = a[2] * b[0] - a[0] * b[2];
-	r[2] = a[0] * b[1] - a[1] * b[0];
-}
-__device__ __forceinline__ double dot3(const double* a, const double* b) { return a[0] * b[0] + (a[1] * b[1] + a[2] * b[2]); }
-__device__ __forceinline__ double norm3(const double* a) { return sqrt(dot3(a, a)); }
-__device__ __forceinline__ void normalize3(double* a) {
-	double r = 1.0 / norm3(a);
-	a[0] *= r; a[1] *= r; a[2] *= r;
-}
-
-// getRotationFromA2B, Riemann.cpp:161-171 (Rodrigues: I + [v]x + (1-c)/s^2 [v]x^2).
-__device__ __forceinline__ void rotation_a2b(const double* A, const double* B, double R[3][3]) {
-	double v[3];
-	cross3(A, B, v);
-	double s = norm3(v);
-	double cc = dot3(A, B);
-	double vx[3][3] = {{0, -v[2], v[1]}, {v[2], 0, -v[0]}, {-v[1], v[0], 0}};
-	double k = (1.0 - cc) / (s * s);
-	double kvx[3][3];
-#pragma unroll
-	for (int i = 0; i < 3; ++i)
-#pragma unroll
-		for (int j = 0; j < 3; ++j) kvx[i][j] = k * vx[i][j];
-#pragma unroll
-	for (int i = 0; i < 3; ++i)
-#pragma unroll
-		for (int j = 0; j < 3; ++j) {
-			double prod = kvx[i][0] * vx[0][j] + kvx[i][1] * vx[1][j] + kvx[i][2] * vx[2][j];
-			R[i][j] = ((i == j ? 1.0 : 0.0) + vx[i][j]) + prod;
-		}
-}
-
-// rotate, Riemann.cpp:154-159.
-__device__ __forceinline__ void rotate(const double R[3][3], double* v) {
-	double x = v[VEL + 0], y = v[VEL + 1], z = v[VEL + 2];
-#pragma unroll
-	for (int i = 0; i < 3; ++i) v[VEL + i] = R[i][0] * x + R[i][1] * y + R[i][2] * z;
-}
-
-// RotatedHartenLaxLeerSolver::solve (Nishikawa & Kitamura 2008), Riemann.cpp:181-244.
-__device__ void rotated_hllc(double* F, const double* Ql, const double* Qr, double a_l2, double a_r2, double gamma, int nd,
-                             int dim) {
-	bool pureHLLC = false, pureHLL = false;
-	double d[3] = {dim == 0 ? 1.0 : 0.0, dim == 1 ? 1.0 : 0.0, dim == 2 ? 1.0 : 0.0};
-	double n1[3] = {Qr[VEL + 0] - Ql[VEL + 0], Qr[VEL + 1] - Ql[VEL + 1], Qr[VEL + 2] - Ql[VEL + 2]};
-	double n2[3] = {0, 0, 0}, t[3];
-	if (n1[dim] < 0)
-		for (int i = 0; i < 3; ++i) n1[i] = -1.0 * n1[i];
-	if (norm3(n1) < 1.0e-6)
-		pureHLLC = true;
-	else {
-		normalize3(n1);
-		cross3(n1, d, t);
-		if (norm3(t) == 0)
-			pureHLL = true;
-		else {
-			cross3(t, n1, n2);
-			if (norm3(n2) == 0)
-				pureHLL = true;
-			else {
-				if (n2[dim] < 0)
-					for (int i = 0; i < 3; ++i) n2[i] = -1.0 * n2[i];
-				normalize3(n2);
-				cross3(n2, d, t);
-				if (norm3(t) == 0) pureHLLC = true;
-			}
-		}
-	}
-	if (!pureHLLC && !pureHLL) {
-		double F1[7] = {0, 0, 0, 0, 0, 0, 0}, F2[7] = {0, 0, 0, 0, 0, 0, 0};
-		double QlR[7], QrR[7], Rm[3][3];
-		for (int i = 0; i < NU; ++i) { QlR[i] = Ql[i]; QrR[i] = Qr[i]; }
-		rotation_a2b(n1, d, Rm);
-		rotate(Rm, QlR);
-		rotate(Rm, QrR);
-		hll(F1, QlR, QrR, a_l2, a_r2, gamma, nd, dim);
-		rotation_a2b(d, n1, Rm);
-		rotate(Rm, QlR);
-		rotate(Rm, QrR);
-		rotate(Rm, F1);
-		rotation_a2b(n2, d, Rm);
-		rotate(Rm, QlR);
-		rotate(Rm, QrR);
-		hllc(F2, QlR, QrR, a_l2, a_r2, gamma, nd, dim);
-		rotation_a2b(d, n2, Rm);
-		rotate(Rm, F2);
-		double w1 = fabs(dot3(d, n1)), w2 = fabs(dot3(d, n2));
-		for (int iu = 0; iu < NU; ++iu) F[iu] = w1 * F1[iu] + w2 * F2[iu];
-	} else if (pureHLL)
-		hll(F, Ql, Qr, a_l2, a_r2, gamma, nd, dim);
-	else
-		hllc(F, Ql, Qr, a_l2, a_r2, gamma, nd, dim);
-}
-
-// ------------------------------------------------------------- hydro faces
-// Ghost position p (< 0 or >= n) along dim -> interior source index and the
-// velocity rule of Grid::applyBCs (Grid.cpp:649-836).  Layer k = 1 is adjacent.
-// A PARTITION face (x-slab decomposition) takes ghost layer k from the
-// neighbour's halo, S.halo_recv [side][k - 1][field][ny * nz], as the
-// reference's ghost cells take the neighbour's Q (Grid.cpp:804-833).
-__device__ __forceinline__ void load_line(const Params& P, const double* __restrict__ Q, const void* halo,
-                                          long long base, long long stride, int n, int dim, int pos, double* q) {
-	int src = pos, cond = -1, side = 0;
-	if (pos < 0) {
-		int k = -pos;
-		cond = P.lbc[dim];
-		src = cond == BC_PERIODIC ? n - k : (cond == BC_REFLECTING ? k : 0);
-	} else if (pos >= n) {
-		int k = pos - n + 1;
-		cond = P.rbc[dim];
-		side = 1;
-		src = cond == BC_PERIODIC ? k - 1 : (cond == BC_REFLECTING ? n - 1 - k : n - 1);
-	}
-	if (cond == BC_PARTITION) {  // x faces only: base = (j + ny k) nx
-		const long long nyz = (long long)P.ny * P.nz, trans = base / P.nx;
-		const int layer = (side ? pos - n + 1 : -pos) - 1;
-		const double* h = static_cast<const double*>(halo) + (long long)(side * 2 + layer) * NU * nyz + trans;
-#pragma unroll
-		for (int f = 0; f < NU; ++f) q[f] = h[(long long)f * nyz];
-		return;
-	}
-	long long id = base + (long long)src * stride;
-#pragma unroll
-	for (int f = 0; f < NU; ++f) q[f] = __ldg(&Q[(long long)f * P.N + id]);
-	if (cond >= 0) {
-		double v = q[VEL + dim];
-		if (cond == BC_INFLOW) {
-			if (side == 0 ? v < 0 : v > 0) q[VEL + dim] = -1.0 * v;
-		} else if (cond == BC_OUTFLOW) {
-			if (side == 0 ? v > 0 : v < 0) q[VEL + dim] = -1.0 * v;
-		} else if (cond == BC_REFLECTING) {
-			q[VEL + dim] = -v;
-		}
-	}
-}
-
-// Hydrodynamics::calcFluxes (Hydro.cpp:91-115) with the reconstruction of
-// Hydro.cpp:44-67: one thread per face along dim; face f lies between line
-// positions f-1 and f.
-__device__ __forceinline__ void b_faces_fp64(const Params& P, const State& S, long long t, int dim);
-__global__ void __launch_bounds__(128) k_faces_fp64(Params P, State S, int dim) {
-	if (TRG_BATCHED && P.batch) {
-		const BatchTable& B = *P.batch;
-		const long long* off = B.face_off[dim];
-		const int g = batch_slot(off, B.G, blockIdx.x * (long long)blockDim.x);
-		const long long lt = blockIdx.x * (long long)blockDim.x + threadIdx.x - off[g];
-		if (lt < B.S[g].nfaces[dim]) b_faces_fp64(B.P[g], B.S[g], lt, dim);
-		return;
-	}
-	const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-	if (t >= S.nfaces[dim]) return;
-	b_faces_fp64(P, S, t, dim);
-}
-__device__ __forceinline__ void b_faces_fp64(const Params& P, const State& S, long long t, int dim) {
-	int n = ncell(P, dim), f;
-	long long base, stride;
-	if (dim == 0) {
-		f = (int)(t % (n + 1));
-		long long rest = t / (n + 1);
-		base = rest * P.nx;
-		stride = 1;
-	} else if (dim == 1) {
-		int i = (int)(t % P.nx);
-		long long rest = t / P.nx;
-		f = (int)(rest % (n + 1));
-		long long k = rest / (n + 1);
-		base = i + (long long)P.nx * P.ny * k;
-		stride = P.nx;
-	} else {
-		long long plane = (long long)P.nx * P.ny;
-		f = (int)(t / plane);
-		base = t % plane;
-		stride = plane;
-	}
-	double Ls[7], Rs[7], Fv[7];
-	if (P.order == 1) {
-		double a[7], b[7], c[7], e[7];
-		load_line(P, S.Q, S.halo_recv, base, stride, n, dim, f - 2, a);
-		load_line(P, S.Q, S.halo_recv, base, stride, n, dim, f - 1, b);
-		load_line(P, S.Q, S.halo_recv, base, stride, n, dim, f, c);
-		load_line(P, S.Q, S.halo_recv, base, stride, n, dim, f + 1, e);
-#pragma unroll
-		for (int iq = 0; iq < NU; ++iq) {
-			// QR of the cell at f-1 and QL of the cell at f (Hydro.cpp:44-50)
-			double sl = limiter(P.limiter, b[iq] - a[iq], c[iq] - b[iq]);
-			Ls[iq] = b[iq] + 0.5 * sl;
-			double sr = limiter(P.limiter, c[iq] - b[iq], e[iq] - c[iq]);
-			Rs[iq] = c[iq] - 0.5 * sr;
-		}
-	} else {
-		load_line(P, S.Q, S.halo_recv, base, stride, n, dim, f - 1, Ls);
-		load_line(P, S.Q, S.halo_recv, base, stride, n, dim, f, Rs);
-	}
-	double a_l2 = P.gamma * Ls[PRE] / Ls[DEN];
-	double a_r2 = P.gamma * Rs[PRE] / Rs[DEN];
-#pragma unroll
-	for (int i = 0; i < NU; ++i) Fv[i] = 0;
-	if (P.riemann == RS_HLLC) hllc(Fv, Ls, Rs, a_l2, a_r2, P.gamma, P.nd, dim);
-	else if (P.riemann == RS_HLL) hll(Fv, Ls, Rs, a_l2, a_r2, P.gamma, P.nd, dim);
-	else rotated_hllc(Fv, Ls, Rs, a_l2, a_r2, P.gamma, P.nd, dim);
-	if (Fv[HII] != Fv[HII]) atomicOr(S.err, ERRB_FLUX);
-	double* Fd = S.F[dim];
-	long long nf = S.nfaces[dim];
-#pragma unroll
-	for (int i = 0; i < NU; ++i) Fd[(long long)i * nf + t] = Fv[i];
-}
+#include "hydro_faces.cuh"
 
 __device__ __forceinline__ void face_ids(const Params& P, const int* ijk, int dim, long long& l, long long& r) {
 	if (dim == 0) {
@@ -2111,18 +1812,30 @@ __global__ void __launch_bounds__(256) k_fb_flags(Params P, State S, double cont
 		if (P.stats_on && lane == leader) atomicAdd(S.stats + TRG_STAT_FP64_CELLS, (unsigned long long)__popc(ballot));
 	}
 }
-// FP64 face fluxes (into S.F) of every listed cell's faces.
+// FP64 face fluxes (into S.F) of every listed cell's faces.  A block takes the
+// faces of one direction, so that its warps run one path and the directions
+// of a short list run side by side.
+template <int DIM, int ND>
+__device__ __forceinline__ void fb_faces_along(const Params& P, const State& S, unsigned n) {
+	const long long nt = (long long)((gridDim.x - DIM + ND - 1) / ND) * blockDim.x;  // threads of this direction
+#pragma unroll 1
+	for (long long t = blockIdx.x / ND * (long long)blockDim.x + threadIdx.x; t < (long long)n * 2; t += nt) {
+		int ijk[3];
+		cell_ijk(P, S.fb_list[t >= n ? t - n : t], ijk);
+		long long fl, fr;
+		face_ids(P, ijk, DIM, fl, fr);
+		one_face<DIM, ND>(P, S, t >= n ? fr : fl);
+	}
+}
 __global__ void __launch_bounds__(128) k_fb_faces(Params P, State S) {
 	const unsigned n = *S.fb_count;
-	for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < (long long)n * 2 * P.nd;
-	     t += (long long)gridDim.x * blockDim.x) {
-		const long long id = S.fb_list[t / (2 * P.nd)];
-		const int k = (int)(t % (2 * P.nd)), dim = k >> 1;
-		int ijk[3];
-		cell_ijk(P, id, ijk);
-		long long fl, fr;
-		face_ids(P, ijk, dim, fl, fr);
-		b_faces_fp64(P, S, (k & 1) ? fr : fl, dim);
+	if (P.nd == 3) {
+		if (blockIdx.x % 3 == 0) fb_faces_along<0, 3>(P, S, n);
+		else if (blockIdx.x % 3 == 1) fb_faces_along<1, 3>(P, S, n);
+		else fb_faces_along<2, 3>(P, S, n);
+	} else {
+		if (blockIdx.x % 2 == 0) fb_faces_along<0, 2>(P, S, n);
+		else fb_faces_along<1, 2>(P, S, n);
 	}
 }
 // FP64 update of every listed cell, U -> U1, with Q of the result.

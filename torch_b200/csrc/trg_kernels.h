@@ -7,7 +7,10 @@
 // reference), fast (FP32 form; FMA and CUDA libm) and fastb (fast, with the
 // batch dispatch, for FP32-form batches)
 #define TRG_FP64_KERNELS \
-	__global__ void k_faces_fp64(Params P, State S, int dim); \
+	__global__ void k_faces_batch_fp64(Params P, State S, int dim); \
+	__global__ void k_faces1_fp64(Params P, State S, FaceGrid G); \
+	__global__ void k_faces2_fp64(Params P, State S, FaceGrid G); \
+	__global__ void k_faces3_fp64(Params P, State S, FaceGrid G); \
 	__global__ void k_hydro_update_fp64(Params P, State S, double h, int sel_base, int sel_out, int mode); \
 	__global__ void k_q_from_u_fp64(Params P, State S, int sel_src, int fix); \
 	__global__ void k_advance_fp64(Params P, State S, double dt); \

@@ -223,4 +223,12 @@ struct BatchTile {
 	int g, tx, ty, pad;  // grid, tile index along x and y
 };
 
+// Launch layout of one grid's face fluxes (k_faces*_fp64): blocks of x faces,
+// of y faces, the rest z faces; a thread of the y and z parts takes `chunk`
+// consecutive faces of a column.
+struct FaceGrid {
+	unsigned bx, by;
+	int chunk;
+};
+
 }  // namespace trg
