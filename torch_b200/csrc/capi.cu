@@ -508,8 +508,13 @@ void thermo_integrate(trg_ctx* c, double h) {
 	c->launches += 3;
 }
 
-void sub_step(trg_ctx* c, double h, bool hasCalculatedHeatFlux, int comp, bool colden_ahead = false) {
+// `last`: the full step's last sub-step.  The updates before it leave Q of the
+// new state for the sub-step that follows; after the last one the FP64 form
+// keeps the Q its sub-step worked on, as the reference does (the FP32 form
+// leaves the new one).
+void sub_step(trg_ctx* c, double h, bool hasCalculatedHeatFlux, int comp, bool last, bool colden_ahead = false) {
 	// Torch::subStep, Torch.cpp:352-364
+	const bool with_q = c->mixed || !last;
 	if (!hasCalculatedHeatFlux) {
 		if (!c->q_fresh) q_from_u(c, 0, 1);
 		c->q_fresh = false;
@@ -558,7 +563,8 @@ void sub_step(trg_ctx* c, double h, bool hasCalculatedHeatFlux, int comp, bool c
 			break;
 		}
 		hydro_fluxes(c);
-		LAUNCH(KF(k_hydro_update_fp64), c->P.N, 256, c->P, c->S, h, 0, 0, 0);
+		LAUNCH(KF(k_hydro_update_fp64), c->P.N, 256, c->P, c->S, h, 0, 0, with_q ? 2 : 0);
+		c->q_fresh = with_q;
 		c->colden_valid = false;
 		break;
 	case COMP_RAD:
@@ -574,14 +580,14 @@ void sub_step(trg_ctx* c, double h, bool hasCalculatedHeatFlux, int comp, bool c
 			c->colden_join_pending = true;
 		}
 		rad_integrate(c, h);
-		// mode 2 (FP32 form): the update also leaves Q of the new state
-		LAUNCH(KF(k_rad_update_fp64), c->P.N, 256, c->P, c->S, h, c->mixed ? 2 : 0);
-		c->q_fresh = c->mixed;
+		// mode 2: the update also leaves Q of the new state
+		LAUNCH(KF(k_rad_update_fp64), c->P.N, 256, c->P, c->S, h, with_q ? 2 : 0);
+		c->q_fresh = with_q;
 		break;
 	default:
 		thermo_integrate(c, h);
-		LAUNCH(KF(k_thermo_update_fp64), c->P.N, 256, c->P, c->S, h, c->mixed ? 2 : 0);
-		c->q_fresh = c->mixed;
+		LAUNCH(KF(k_thermo_update_fp64), c->P.N, 256, c->P, c->S, h, with_q ? 2 : 0);
+		c->q_fresh = with_q;
 		break;
 	}
 }
@@ -591,8 +597,7 @@ void hydro_step(trg_ctx* c) {
 	// saved state W is the untouched U; the predictor writes U1.
 	c->colden_valid = false;
 	hydro_fluxes(c);
-	LAUNCH(KF(k_hydro_update_fp64), c->P.N, 256, c->P, c->S, 0.5, 0, 1, 0);
-	q_from_u(c, 1, 0);
+	LAUNCH(KF(k_hydro_update_fp64), c->P.N, 256, c->P, c->S, 0.5, 0, 1, 3);
 	hydro_fluxes(c);
 	LAUNCH(KF(k_hydro_update_fp64), c->P.N, 256, c->P, c->S, 1.0, 0, 0, 0);
 }
@@ -626,9 +631,12 @@ void time_step(trg_ctx* c, double dt_next) {
 		first_cell = c->hs.first_nonwind_cell;
 		c->rad_once_pending = 0;
 	}
-	LAUNCH_SCALAR(KF(k_dt_reset), c->P, c->S);
-	LAUNCH(KF(k_dt_reduce_fp64), c->P.N, 256, c->P, c->S, first_cell);
+	// the reduction's last block takes the step, unless the minima of the other
+	// slabs come in between
+	const DtEnd end{c->xfn ? 0 : 1, step, dt_next};
+	LAUNCH(KF(k_dt_reduce_fp64), c->P.N, 256, c->P, c->S, first_cell, end);
 	if (c->cons_on) cons_record(c, true);
+	if (end.on) return;
 	dt_exchange(c);
 	LAUNCH_SCALAR(KF(k_dt_finalize), c->P, c->S, dt_next, 0, step);
 }
@@ -642,7 +650,6 @@ void enqueue_full_step_fp32(trg_ctx* c, double dt_next) {
 	if (!c->first_time) dt_exchange(c);
 	LAUNCH_SCALAR(KF(k_dt_finalize), c->P, c->S, dt_next, c->first_time, step);
 	c->first_time = 0;
-	LAUNCH_SCALAR(KF(k_dt_reset), c->P, c->S);
 	auto stage = [&](int st, const float* Uq, const float* Ub, float* Uo) {
 		halo_exchange(c, Uq, true);
 		cudaEvent_t ea = nullptr, eb = nullptr;
@@ -653,7 +660,6 @@ void enqueue_full_step_fp32(trg_ctx* c, double dt_next) {
 	};
 	stage(1, c->U32, c->U32, c->U32s);
 	stage(2, c->U32s, c->U32, c->U32);
-	LAUNCH_SCALAR(KF(k_time_advance), c->P, c->S);
 	c->steps++;
 }
 
@@ -718,10 +724,9 @@ void enqueue_full_step(trg_ctx* c, double dt_next) {
 					}
 				}
 			}
-			sub_step(c, hs[k], k == 0, seq[k], ahead);
+			sub_step(c, hs[k], k == 0, seq[k], k == ns - 1, ahead);
 		}
 	}
-	LAUNCH_SCALAR(KF(k_time_advance), c->P, c->S);
 	c->steps++;
 }
 
@@ -1107,10 +1112,11 @@ int trg_component(trg_ctx* c, int comp, int phase, double dt, double* out) {
 			first_cell = c->hs.first_nonwind_cell;
 			c->rad_once_pending = 0;
 		}
-		LAUNCH(KF(k_dt_reduce_fp64), c->P.N, 256, c->P, c->S, first_cell);
+		LAUNCH(KF(k_dt_reduce_fp64), c->P.N, 256, c->P, c->S, first_cell, (DtEnd{0, -1, 0.0}));
 		double mins[3];
 		CUDA_TRY(cudaMemcpyAsync(mins, c->S.scal + 2, sizeof(mins), cudaMemcpyDeviceToHost, c->stream));
 		CUDA_TRY(cudaStreamSynchronize(c->stream));
+		LAUNCH_SCALAR(KF(k_dt_reset), c->P, c->S);
 		double v = c->P.dt_max;
 		if (comp == TRG_COMP_HYDRO) v = mins[0] < v ? mins[0] : v;
 		else if (comp == TRG_COMP_RAD) v = (c->P.star_on && mins[1] < v) ? mins[1] : v;
@@ -1247,6 +1253,9 @@ int trg_checkpoint_load(trg_ctx* c, const void* buf, long long bytes) {
 	}
 	if (c->fp32) CUDA_TRY(cudaMemcpy(c->U32, p, 7 * N * sizeof(float), cudaMemcpyHostToDevice));
 	CUDA_TRY(cudaMemcpy(c->S.scal, h.scal, sizeof(h.scal), cudaMemcpyHostToDevice));
+	// the time-step minima start from dt_max (the hydro-only FP32 form's hold
+	// the next step's limit), whatever an earlier build left in the blob
+	if (!c->fp32) LAUNCH_SCALAR(KF(k_dt_reset), c->P, c->S);
 	CUDA_TRY(cudaMemset(c->S.UDOT, 0, 7 * N * sizeof(double)));
 	c->q_fresh = h.q_fresh != 0;
 	c->colden_valid = false;

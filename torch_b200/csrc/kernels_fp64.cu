@@ -88,17 +88,23 @@ __device__ __forceinline__ void hydro_udot(const Params& P, const State& S, long
 	}
 }
 
-// globalQfromU + fixPrimitives + checkValues of a cell whose new conserved
-// state u the caller has in registers (the FP32 form's updates finish with
-// it, so that the next sub-step's Q pass is skipped).  Q fields of velocity
-// components beyond nd are left as they are, as QfromU leaves them.
-__device__ __forceinline__ void store_fixed_q(const Params& P, const State& S, long long id, const double* u) {
+// globalQfromU of a cell whose new conserved state u the caller has in
+// registers, with FIX also fixPrimitives and checkValues: an update that
+// another sub-step follows finishes with it, so that the next Q pass is
+// skipped.  Q fields of velocity components beyond nd are left as they are, as
+// QfromU leaves them.  (Torch::checkValues runs where Q was just rebuilt with
+// floors; the reference does not check the RK2 predictor's Q.)
+template <bool FIX>
+__device__ __forceinline__ void store_q(const Params& P, const State& S, long long id, const double* u) {
 	double q[7] = {0, 0, 0, 0, 0, 0, 0};
 	QfromU(q, u, P.gamma, P.nd);
-	fix_primitives(P, q, u[DEN]);
-	bool bad = q[DEN] == 0 || q[PRE] == 0;
+	if (FIX) {
+		fix_primitives(P, q, u[DEN]);
+		bool bad = q[DEN] == 0 || q[PRE] == 0;
 #pragma unroll
-	for (int i = 0; i < NU; ++i) bad |= (u[i] != u[i]) || isinf(u[i]);
+		for (int i = 0; i < NU; ++i) bad |= (u[i] != u[i]) || isinf(u[i]);
+		if (bad) atomicOr(S.err, ERRB_NAN);
+	}
 	FLD(S.Q, DEN, id) = q[DEN];
 	FLD(S.Q, PRE, id) = q[PRE];
 	FLD(S.Q, HII, id) = q[HII];
@@ -106,13 +112,15 @@ __device__ __forceinline__ void store_fixed_q(const Params& P, const State& S, l
 #pragma unroll
 	for (int k = 0; k < 3; ++k)
 		if (k < P.nd) FLD(S.Q, VEL + k, id) = q[VEL + k];
-	if (bad) atomicOr(S.err, ERRB_NAN);
 }
 
 // Hydro update: UDOT from the face fluxes, then Fluid::advSolution (Fluid.cpp:80-87)
 // from Ubase and Fluid::fixSolution, written to Uout (may alias Ubase); the
 // selectors pick S.U (0) or S.U1 (1).
-// mode 1 accumulates UDOT into S.UDOT instead (component-phase interface).
+// mode 1 accumulates UDOT into S.UDOT instead (component-phase interface);
+// modes 2 and 3 also leave Q of the new state, as globalQfromU would form it in
+// a pass of its own (168 B per cell saved): 2 with floors and checks, for a
+// sub-step that another one follows, 3 without, for the RK2 corrector.
 __device__ __forceinline__ void b_hydro_update_fp64(const Params& P, const State& S, long long id, double h, int sel_base,
                                                     int sel_out, int mode) {
 	const double* Ubase = sel_base ? S.U1 : S.U;
@@ -133,7 +141,8 @@ __device__ __forceinline__ void b_hydro_update_fp64(const Params& P, const State
 	if (!fix_solution(P, u)) atomicOr(S.err, ERRB_NAN);
 #pragma unroll
 	for (int i = 0; i < NU; ++i) FLD(Uout, i, id) = u[i];
-	if (mode == 2) store_fixed_q(P, S, id, u);
+	if (mode == 2) store_q<true>(P, S, id, u);
+	else if (mode == 3) store_q<false>(P, S, id, u);
 }
 __global__ void __launch_bounds__(256) k_hydro_update_fp64(Params P, State S, double h, int sel_base, int sel_out,
                                                           int mode) {
@@ -1104,7 +1113,7 @@ __device__ __forceinline__ void b_rad_update_fp64(const Params& P, const State& 
 	if (!fix_solution(P, u)) atomicOr(S.err, ERRB_NAN);
 #pragma unroll
 	for (int i = 0; i < NU; ++i) FLD(S.U, i, id) = u[i];
-	if (mode == 2) store_fixed_q(P, S, id, u);
+	if (mode == 2) store_q<true>(P, S, id, u);
 }
 __global__ void __launch_bounds__(256) k_rad_update_fp64(Params P, State S, double h, int mode) {
 	if (TRG_BATCHED && P.batch) {
@@ -1501,7 +1510,7 @@ __device__ __forceinline__ void b_thermo_update_fp64(const Params& P, const Stat
 	if (!fix_solution(P, u)) atomicOr(S.err, ERRB_NAN);
 #pragma unroll
 	for (int i = 0; i < NU; ++i) FLD(S.U, i, id) = u[i];
-	if (mode == 2) store_fixed_q(P, S, id, u);
+	if (mode == 2) store_q<true>(P, S, id, u);
 }
 __global__ void __launch_bounds__(256) k_thermo_update_fp64(Params P, State S, double h, int mode) {
 	if (TRG_BATCHED && P.batch) {
@@ -1583,18 +1592,32 @@ __device__ __forceinline__ double block_min(double v) {
 // With cons_part set (single grids only) the pass also forms the block's
 // partial of the global FP64 mass and energy sums of the state (U), the
 // conservation check of the step.
+//
+// The last block of a grid to finish (end.on) also takes the time step from
+// the minima, so that no launch of its own follows (a slab's minima first go
+// through the exchange: end.on = 0 and k_dt_finalize).
+__device__ __forceinline__ void b_dt_finalize(const Params& P, const State& S, double dt_next, int first_time, int step);
 __device__ __forceinline__ void b_dt_reduce_fp64(const Params& P, const State& S, long long id, long long first_cell,
                                                  double* cons_part);
-__global__ void __launch_bounds__(256) k_dt_reduce_fp64(Params P, State S, long long first_cell) {
+__device__ __forceinline__ void dt_end(const Params& P, const State& S, const DtEnd& end, unsigned nblocks) {
+	if (!end.on || threadIdx.x != 0) return;
+	__threadfence();  // this block's minima before its count
+	if (atomicInc(reinterpret_cast<unsigned*>(S.scal + SCAL_BLOCKS), nblocks - 1) != nblocks - 1) return;
+	__threadfence();
+	b_dt_finalize(P, S, end.dt_next, 0, end.step);
+}
+__global__ void __launch_bounds__(256) k_dt_reduce_fp64(Params P, State S, long long first_cell, DtEnd end) {
 	if (TRG_BATCHED && P.batch) {
 		// grid ranges are padded to whole blocks: the block reduction stays within one grid
 		const BatchTable& B = *P.batch;
 		const int g = batch_slot(B.cell_off, B.G, blockIdx.x * (long long)blockDim.x);
 		const long long lid = blockIdx.x * (long long)blockDim.x + threadIdx.x - B.cell_off[g];
 		b_dt_reduce_fp64(B.P[g], B.S[g], lid, first_cell >= 0 ? B.first_cell[g] : -1, nullptr);
+		dt_end(B.P[g], B.S[g], end, (unsigned)((B.cell_off[g + 1] - B.cell_off[g]) / blockDim.x));
 		return;
 	}
 	b_dt_reduce_fp64(P, S, blockIdx.x * (long long)blockDim.x + threadIdx.x, first_cell, S.cons_part);
+	dt_end(P, S, end, gridDim.x);
 }
 __device__ __forceinline__ void b_dt_reduce_fp64(const Params& P, const State& S, long long id, long long first_cell,
                                                  double* cons_part) {
@@ -1675,8 +1698,34 @@ __device__ __forceinline__ void b_dt_reduce_fp64(const Params& P, const State& S
 	}
 }
 
-// Torch::calculateTimeStep + the dt of Torch::fullStep (Torch.cpp:304-339, :394).
-__device__ __forceinline__ void b_dt_finalize(const Params& P, const State& S, double dt_next, int first_time, int step);
+// Torch::calculateTimeStep + the dt of Torch::fullStep (Torch.cpp:304-339,
+// :394).  The minima are taken up here, so they start again from dt_max for
+// the next reduction, and the run's time moves on: nothing in the step reads
+// either, and neither needs a launch of its own.
+__device__ __forceinline__ void b_dt_reset(const Params& P, const State& S) {
+	unsigned long long big = (unsigned long long)__double_as_longlong(P.dt_max);
+	unsigned long long* slots = reinterpret_cast<unsigned long long*>(S.scal + 2);
+	slots[0] = big;
+	slots[1] = big;
+	slots[2] = big;
+}
+__device__ __forceinline__ void b_dt_finalize(const Params& P, const State& S, double dt_next, int first_time, int step) {
+	double dt;
+	if (first_time) {
+		dt = P.dt_max * 1.0e-20;
+	} else {
+		double dt_hydro = smin(__ldcg(&S.scal[2]), P.dt_max);
+		double dt_rad = dt_hydro, dt_thermo = dt_hydro;
+		if (P.radiation_on) dt_rad = P.star_on ? smin(P.dt_max, __ldcg(&S.scal[3])) : P.dt_max;
+		if (P.cooling_on) dt_thermo = smin(P.dt_max, __ldcg(&S.scal[4]));
+		dt = smin(smin(dt_hydro, dt_rad), dt_thermo);
+	}
+	dt = smin(dt_next, dt);
+	S.scal[0] = dt;
+	S.scal[1] += dt;
+	b_dt_reset(P, S);
+	if (S.dt_hist && step >= 0) S.dt_hist[step] = dt;
+}
 __global__ void k_dt_finalize(Params P, State S, double dt_next, int first_time, int step) {
 	if (TRG_BATCHED && P.batch) {
 		const int g = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1685,46 +1734,9 @@ __global__ void k_dt_finalize(Params P, State S, double dt_next, int first_time,
 	}
 	b_dt_finalize(P, S, dt_next, first_time, step);
 }
-__device__ __forceinline__ void b_dt_finalize(const Params& P, const State& S, double dt_next, int first_time, int step) {
-	double dt;
-	if (first_time) {
-		dt = P.dt_max * 1.0e-20;
-	} else {
-		double dt_hydro = smin(S.scal[2], P.dt_max);
-		double dt_rad = dt_hydro, dt_thermo = dt_hydro;
-		if (P.radiation_on) dt_rad = P.star_on ? smin(P.dt_max, S.scal[3]) : P.dt_max;
-		if (P.cooling_on) dt_thermo = smin(P.dt_max, S.scal[4]);
-		dt = smin(smin(dt_hydro, dt_rad), dt_thermo);
-	}
-	dt = smin(dt_next, dt);
-	S.scal[0] = dt;
-	if (S.dt_hist && step >= 0) S.dt_hist[step] = dt;
-}
-
-__global__ void k_time_advance(Params P, State S) {
-	if (TRG_BATCHED && P.batch) {
-		const int g = blockIdx.x * blockDim.x + threadIdx.x;
-		if (g < P.batch->G) P.batch->S[g].scal[1] += P.batch->S[g].scal[0];
-		return;
-	}
-	S.scal[1] += S.scal[0];
-}
-
-__device__ __forceinline__ void b_dt_reset(const Params& P, const State& S) {
-	unsigned long long big = (unsigned long long)__double_as_longlong(P.dt_max);
-	unsigned long long* slots = reinterpret_cast<unsigned long long*>(S.scal + 2);
-	slots[0] = big;
-	slots[1] = big;
-	slots[2] = big;
-}
-__global__ void k_dt_reset(Params P, State S) {
-	if (TRG_BATCHED && P.batch) {
-		const int g = blockIdx.x * blockDim.x + threadIdx.x;
-		if (g < P.batch->G) b_dt_reset(P.batch->P[g], P.batch->S[g]);
-		return;
-	}
-	b_dt_reset(P, S);
-}
+// The minima from dt_max again, after a reduction whose minima the host read
+// and after a restored checkpoint (single grids).
+__global__ void k_dt_reset(Params P, State S) { b_dt_reset(P, S); }
 
 // ------------------------------------------- FP64 fallback of the FP32 form
 // A hydro sub-step of the FP32 form keeps FP64 arithmetic for the cells whose

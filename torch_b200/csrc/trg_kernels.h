@@ -43,9 +43,8 @@
 	__global__ void k_fb_flags(Params P, State S, double contrast); \
 	__global__ void k_fb_faces(Params P, State S); \
 	__global__ void k_fb_update(Params P, State S, double h); \
-	__global__ void k_dt_reduce_fp64(Params P, State S, long long first_cell); \
+	__global__ void k_dt_reduce_fp64(Params P, State S, long long first_cell, DtEnd end); \
 	__global__ void k_dt_finalize(Params P, State S, double dt_next, int first_time, int step); \
-	__global__ void k_time_advance(Params P, State S); \
 	__global__ void k_dt_reset(Params P, State S);
 
 namespace trg {

@@ -58,6 +58,8 @@ constexpr int LCAND_MAX = 1 << 21;
 // persistent grid of the learned-start inference (4 CTAs per SM of a B200)
 constexpr int INFER_CTAS = 148 * 4;
 
+constexpr int SCAL_BLOCKS = 5;  // State::scal
+
 // Planes per CTA of the FP32 form's fallback flag pass (k_fb_flags).
 constexpr int FB_ZCHUNK = 16;
 
@@ -146,7 +148,9 @@ struct State {
 	long long nfaces[3];
 	const Tables* tables;
 	unsigned* err;
-	// scalars: [0] dt, [1] time, [2..4] per-component dt minima (as uint64 bits)
+	// scalars: [0] dt, [1] time, [2..4] per-component dt minima (as uint64
+	// bits), [SCAL_BLOCKS] the reduction's count of finished blocks (unsigned,
+	// 0 between launches)
 	double* scal;
 	double* dt_hist;
 	// diagnostic counters, TRG_STAT_* indices of the C ABI header
@@ -221,6 +225,13 @@ struct BatchTable {
 };
 struct BatchTile {
 	int g, tx, ty, pad;  // grid, tile index along x and y
+};
+
+// What the time-step reduction does when its last block is done: nothing, or
+// (on) the time step itself, at most dt_next, recorded as step `step`.
+struct DtEnd {
+	int on, step;
+	double dt_next;
 };
 
 // Launch layout of one grid's face fluxes (k_faces*_fp64): blocks of x faces,
