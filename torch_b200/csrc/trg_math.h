@@ -148,7 +148,39 @@ TRG_MATH_FN double trg_exp_dd(double xh, double xl) {
 	return (z - grid) * 0x1p-1074;
 }
 
-TRG_MATH_FN double trg_exp(double x) { return trg_exp_dd(x, 0.0); }
+/* exp(x) rounded to nearest, by Ziv's strategy (A. Ziv, "Fast evaluation of
+   elementary mathematical functions with correctly rounded last bit", ACM
+   TOMS 17, 1991): a shorter evaluation whose error is below 2^-66 of the
+   result's leading part, taken where adding and subtracting that bound rounds
+   to the same double (all but about 2^-12 of the arguments), else
+   trg_exp_dd.  The shorter one is what a dependent chain of exponentials
+   waits for: 14 dependent operations instead of 43.
+   x = k ln2/128 + r as there; exp(r) - 1 = rh + lo, lo = r^2 (1/2 + r (1/6 +
+   r/24 + r^2 (1/120 + r/720))) + rl (truncated at 2^-71); times the table's
+   th + tl as s1 + w with th + th rh = s1 + e1 exactly (two-product, two-sum). */
+TRG_MATH_FN double trg_exp(double x) {
+	if (!(x > -708.0 && x < 709.0)) return trg_exp_dd(x, 0.0);
+	const double kshift = fma(x, TRG_EXP_INV_LN2_128, 0x1.8p52);
+	const double kd = kshift - 0x1.8p52;
+	const int k = (int)(uint32_t)trg_double_to_bits(kshift);
+	const int j = k & 127, ex = (k - j) / 128;
+	const double th = TRG_TAB(trg_exp_tab, 2 * j), tl = TRG_TAB(trg_exp_tab, 2 * j + 1);
+	const double t1 = fma(-kd, TRG_EXP_LN2_128_1, x); /* exact */
+	double p, pe, rh, rl;
+	trg_two_prod(kd, TRG_EXP_LN2_128_2, &p, &pe);
+	trg_two_sum(t1, -p, &rh, &rl);
+	rl = rl - fma(kd, TRG_EXP_LN2_128_3, pe);
+	const double r2 = rh * rh;
+	const double q = fma(r2, fma(rh, 1.0 / 720.0, 1.0 / 120.0), fma(rh, 1.0 / 24.0, 1.0 / 6.0));
+	const double lo = fma(r2, fma(rh, q, 0.5), rl);
+	double m, me;
+	trg_two_prod(th, rh, &m, &me);
+	const double s1 = th + m, e1 = m - (s1 - th);
+	const double w = (e1 + me) + fma(th, lo, fma(tl, rh, tl));
+	const double up = s1 + (w + 0x1p-65), down = s1 + (w - 0x1p-65);
+	if (up != down) return trg_exp_dd(x, 0.0);
+	return up * trg_pow2i(ex);
+}
 
 /* log(x) as a double-double hi + lo (hi the rounded result), x > 0 finite. */
 TRG_MATH_FN void trg_log_dd(double x, double* hi, double* lo) {
