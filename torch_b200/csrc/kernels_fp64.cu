@@ -829,10 +829,23 @@ __global__ void __launch_bounds__(128) k_batch_learned_infer(Params Pv, State Sv
 // recombination rate and the collisional ionisation rate at the cell's
 // temperature, and x_HII; with `init` also the fixed path length and shell
 // volume.  One parallel pass before each sweep (single grids only).
+__device__ __forceinline__ void b_rad_sweep_prep(const Params& P, const State& S, const int* __restrict__ cells, int t,
+                                                 int init);
 __global__ void __launch_bounds__(256) k_rad_sweep_prep(Params P, State S, const int* __restrict__ cells, int n,
                                                          int init) {
+	if (TRG_BATCHED && P.batch) {  // grids whose sweep is a chain (no learned start)
+		const BatchTable& B = *P.batch;
+		const int g = batch_slot(B.cell_off, B.G, blockIdx.x * (long long)blockDim.x);
+		const long long lt = blockIdx.x * (long long)blockDim.x + threadIdx.x - B.cell_off[g];
+		const State& Sg = B.S[g];
+		if (lt < Sg.sw_rad_n) b_rad_sweep_prep(B.P[g], Sg, Sg.chain_rad->cells, (int)lt, init);
+		return;
+	}
 	const int t = blockIdx.x * blockDim.x + threadIdx.x;
-	if (t >= n) return;
+	if (t < n) b_rad_sweep_prep(P, S, cells, t, init);
+}
+__device__ __forceinline__ void b_rad_sweep_prep(const Params& P, const State& S, const int* __restrict__ cells, int t,
+                                                 int init) {
 	const long long id = cells[t];
 	const long long sn = S.sw_rad_n;
 	double* sw = S.sw_rad + t;
@@ -1177,6 +1190,37 @@ __device__ __forceinline__ double th_cooling(const Params& P, const State& S, do
 	return r;
 }
 
+// Thermodynamics::updateColDen's interpolation (Thermodynamics.cpp:339-363)
+// from the upwind neighbours' column densities (0: not read).
+__device__ __forceinline__ double colden_interp(const double* colden, const double* w0) {
+#ifdef TRG_FAST_MATH
+	// The weighted harmonic mean sum(w0) / sum(w0 / c) over the non-zero c;
+	// numerator and denominator scaled by the product of those c take one
+	// division (per-neighbour divisions where that product would overflow).
+	double m[4];
+	for (int i = 0; i < 4; ++i) m[i] = colden[i] == 0 ? 1.0 : colden[i];
+	const double m01 = m[0] * m[1], m23 = m[2] * m[3], prod = m01 * m23;
+	if (prod < 1.0e300) {
+		const double p[4] = {m[1] * m23, m[0] * m23, m[3] * m01, m[2] * m01};
+		double num = 0, den = 0;
+		for (int i = 0; i < 4; ++i)
+			if (colden[i] != 0) {
+				num += w0[i];
+				den += w0[i] * p[i];
+			}
+		return den != 0 ? num * prod / den : 0.0;
+	}
+#endif
+	double w[4], newcolden = 0.0;
+	for (int i = 0; i < 4; ++i) w[i] = colden[i] == 0 ? 0 : w0[i] / colden[i];
+	double sum_w = w[0] + w[1] + w[2] + w[3];
+	for (int i = 0; i < 4 && sum_w != 0; ++i) {
+		w[i] = w[i] / sum_w;
+		newcolden += w[i] * colden[i];
+	}
+	return newcolden;
+}
+
 // One shell of Thermodynamics::rayTrace / updateColDen (Thermodynamics.cpp:339-417).
 // `own`: the cell's ds rho / m_H in the sweep-ordered array, or null.
 __device__ __forceinline__ void b_colden_shell_fp64(const Params& P, const State& S, long long id,
@@ -1195,64 +1239,37 @@ __device__ __forceinline__ void b_colden_shell_fp64(const Params& P, const State
 	sweep_wait();
 	double newcolden = 0.0;
 	if (inner) {
-		double colden[4] = {0, 0, 0, 0}, w[4];
-#ifdef TRG_FAST_MATH
+		double colden[4] = {0, 0, 0, 0};
 		for (int i = 0; i < 4; ++i)
 			if (src[i]) {
 				const double2 c = __ldcg(src[i]);  // COL_DEN, DCOL_DEN
 				colden[i] = c.x + c.y;
 			}
-		// The interpolation is the weighted harmonic mean sum(w0) / sum(w0 / c)
-		// over the non-zero c; numerator and denominator scaled by the product
-		// of those c take one division (per-neighbour divisions where that
-		// product would overflow).
-		double m[4];
-		for (int i = 0; i < 4; ++i) m[i] = colden[i] == 0 ? 1.0 : colden[i];
-		const double m01 = m[0] * m[1], m23 = m[2] * m[3], prod = m01 * m23;
-		if (prod < 1.0e300) {
-			const double p[4] = {m[1] * m23, m[0] * m23, m[3] * m01, m[2] * m01};
-			double num = 0, den = 0;
-			for (int i = 0; i < 4; ++i)
-				if (colden[i] != 0) {
-					num += w0[i];
-					den += w0[i] * p[i];
-				}
-			newcolden = den != 0 ? num * prod / den : 0.0;
-		} else {
-			for (int i = 0; i < 4; ++i) w[i] = colden[i] == 0 ? 0 : w0[i] / colden[i];
-			double sum_w = w[0] + w[1] + w[2] + w[3];
-			for (int i = 0; i < 4 && sum_w != 0; ++i) {
-				w[i] = w[i] / sum_w;
-				newcolden += w[i] * colden[i];
-			}
-		}
-#else
-		for (int i = 0; i < 4; ++i) {
-			if (src[i]) {
-				const double2 c = __ldcg(src[i]);  // COL_DEN, DCOL_DEN
-				colden[i] = c.x + c.y;
-			}
-			w[i] = colden[i] == 0 ? 0 : w0[i] / colden[i];
-		}
-		double sum_w = w[0] + w[1] + w[2] + w[3];
-		for (int i = 0; i < 4 && sum_w != 0; ++i) {
-			w[i] = w[i] / sum_w;
-			newcolden += w[i] * colden[i];
-		}
-#endif
+		newcolden = colden_interp(colden, w0);
 	}
 	reinterpret_cast<double2*>(S.T + id * 2)[0] = make_double2(newcolden, dcolden);
 }
 // The cell's own column density of the sweep in sweep order (S.sw_col):
 // ds rho / m_H, as b_colden_shell_fp64 forms it; with `init` also the fixed
 // path lengths.  One parallel pass before each column-density sweep.
-__global__ void __launch_bounds__(256) k_colden_sweep_prep(Params P, State S, const int* __restrict__ cells, int n,
-                                                            int init) {
-	const int t = blockIdx.x * blockDim.x + threadIdx.x;
-	if (t >= n) return;
+__device__ __forceinline__ void b_colden_sweep_prep(const Params& P, const State& S, const int* __restrict__ cells,
+                                                    int t, int init) {
 	const long long id = cells[t];
 	if (init) S.sw_col[S.sw_col_n + t] = S.ds[id];
 	S.sw_col[t] = (FLD(S.Q, DEN, id) / P.hydrogenMass) * S.sw_col[S.sw_col_n + t];
+}
+__global__ void __launch_bounds__(256) k_colden_sweep_prep(Params P, State S, const int* __restrict__ cells, int n,
+                                                            int init) {
+	if (TRG_BATCHED && P.batch) {  // grids whose sweep is a chain
+		const BatchTable& B = *P.batch;
+		const int g = batch_slot(B.cell_off, B.G, blockIdx.x * (long long)blockDim.x);
+		const long long lt = blockIdx.x * (long long)blockDim.x + threadIdx.x - B.cell_off[g];
+		const State& Sg = B.S[g];
+		if (lt < Sg.sw_col_n) b_colden_sweep_prep(B.P[g], Sg, Sg.chain_col->cells, (int)lt, init);
+		return;
+	}
+	const int t = blockIdx.x * blockDim.x + threadIdx.x;
+	if (t < n) b_colden_sweep_prep(P, S, cells, t, init);
 }
 __global__ void __launch_bounds__(128) k_colden_shell_sw(Params P, State S, const int* __restrict__ cells, int count,
                                                           long long off) {
@@ -1270,6 +1287,8 @@ __global__ void __launch_bounds__(128) k_colden_shell_fp64(Params P, State S, co
 	}
 	b_colden_shell_fp64(P, S, cells[t]);
 }
+
+#include "sweep_chain.cuh"
 
 // Thermodynamics::preTimeStepCalculations rates, Thermodynamics.cpp:224-263, non-wind cells.
 __device__ __forceinline__ void b_thermo_rates_fp64(const Params& P, const State& S, long long id) {

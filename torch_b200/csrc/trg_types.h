@@ -78,6 +78,22 @@ struct Tables {
 // after initialise(), Star, Thermodynamics constants).
 struct BatchTable;
 
+// One grid's causal sweep as a chain of shells walked by one CTA
+// (sweep_chain.cuh): the sweep list cut into shells by off[nshell + 1], and by
+// position in the list the ring places of the cell's upwind neighbours and
+// their weights [4][n].
+struct alignas(16) ChainSlots {
+	int x, y, z, w;
+};
+struct SweepChain {
+	int nshell, n, maxshell;
+	const int* cells;
+	const int* off;
+	const ChainSlots* slot;
+	const double* w;
+};
+constexpr int CHAIN_GROUP = 256;  // most threads of one of the two groups that take a chain's shells in turn
+
 struct Params {
 	int nd, nx, ny, nz;
 	long long N;
@@ -198,6 +214,9 @@ struct State {
 	long long sw_rad_n;
 	double* sw_col;
 	long long sw_col_n;
+	// the two sweeps' chain tables (device structs; null: a launch per shell)
+	const SweepChain* chain_rad;
+	const SweepChain* chain_col;
 	// global FP64 mass and energy sums (null: off): the time-step reduction
 	// also leaves per-block double-double partials of sum(rho V) and sum(E V)
 	// here, 4 doubles per 256-cell block (mass hi, lo, energy hi, lo)
