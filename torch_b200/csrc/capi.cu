@@ -8,6 +8,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -885,14 +886,30 @@ namespace trg {
 const Params& ctx_params(const trg_ctx* c) { return c->P; }
 State ctx_state(const trg_ctx* c) { return c->S; }
 int ctx_device(const trg_ctx* c) { return c->raw.device; }
+// Planes per CTA of the FP32 hydro pass on this grid: a CTA's time is its
+// planes and about 3.5 more (the planes before its first are loaded and one of
+// them computed), and two CTAs fit on an SM, so the grid takes
+// ceil(CTAs / 2 SMs) times that (a wave that is 6% over still ends with the
+// others).  Measured per launch against a fixed least depth of 16 (64 CTAs on
+// 148 SMs at 64^3): 32^3 137 -> 31 us, 64^3 142 -> 57, 75^3 143 -> 96 (FP64 state
+// 198 -> 138), 96^3 154 -> 128, 100^3 (FP64 state) 381 -> 282; the choice is within
+// 4% of the best depth on each.
 int ctx_fp32_zchunk(const trg_ctx* c) {
 	int sms = 148;
 	cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->raw.device);
-	long long tiles = (long long)((c->P.nx + 31) / 32) * ((c->P.ny + 7) / 8);
-	long long nchunks = (4LL * 2 * sms + tiles - 1) / tiles;
-	if (nchunks < 1) nchunks = 1;
-	int zc = (int)((c->P.nz + nchunks - 1) / nchunks);
-	return zc < 16 ? 16 : zc;
+	const long long tiles = (long long)((c->P.nx + 31) / 32) * ((c->P.ny + 7) / 8);
+	int best = c->P.nz;
+	double best_cost = 1e300;
+	for (int chunks = 1; chunks <= c->P.nz; ++chunks) {
+		const int zc = (c->P.nz + chunks - 1) / chunks;
+		const long long ctas = tiles * ((c->P.nz + zc - 1) / zc);
+		const double cost = std::max(1.0, std::ceil((double)ctas / (2.0 * sms) - 0.06)) * (zc + 3.5);
+		if (cost < best_cost) {
+			best_cost = cost;
+			best = zc;
+		}
+	}
+	return best;
 }
 int ctx_fail(trg_ctx* c, int code, const std::string& msg) { return set_error(c, code, msg); }
 // a slab with partition faces and no exchange hook yet
@@ -1008,7 +1025,6 @@ int create_impl(const trg_params* p, const SlabSpec* slab, const double* den, co
 		if (c->P.nd < 2) return set_error(c, TRG_ERR_ARG, "the FP32 form needs a 2-D or 3-D grid");
 		c->fp32 = true;
 		c->fastk = 1;
-		// z chunk per CTA: about four waves of two 256-thread CTAs per SM
 		c->zchunk = ctx_fp32_zchunk(c);
 		if ((rc = dalloc(c, &c->U32, 7 * N)) || (rc = dalloc(c, &c->U32s, 7 * N))) return rc;
 		LAUNCH(k_f64_to_f32, 7 * N, 256, c->P, S.U, c->U32);
