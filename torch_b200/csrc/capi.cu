@@ -69,6 +69,9 @@ struct trg_ctx {
 	// current U (written by the FP32 hydro sub-step), so the next
 	// globalQfromU + fixPrimitives pass can be skipped
 	bool q_fresh = false;
+	// FP32 form with radiation/cooling: U has come out of an update since the
+	// host last set it, so every field is within its floors
+	bool u_fixed = false;
 	// the column densities of the thermodynamics depend on the density alone,
 	// which only hydro sub-steps change: a second sweep with no hydro sub-step
 	// since the last one would recompute the same values and is skipped
@@ -627,15 +630,26 @@ void sub_step(trg_ctx* c, double h, bool hasCalculatedHeatFlux, int comp, bool l
 		}
 		rad_integrate(c, h);
 		// mode 2: the update also leaves Q of the new state
-		LAUNCH(KF(k_rad_update_fp64), c->P.N, 256, c->P, c->S, h, with_q ? 2 : 0);
+		if (c->u_fixed && c->P.star_on && c->P.coupling == CP_NEQ)
+			LAUNCH(KF(k_rad_update_lean), c->P.N, 256, c->P, c->S, h);
+		else
+			LAUNCH(KF(k_rad_update_fp64), c->P.N, 256, c->P, c->S, h, with_q ? 2 : 0);
 		c->q_fresh = with_q;
 		break;
 	default:
-		thermo_integrate(c, h);
-		LAUNCH(KF(k_thermo_update_fp64), c->P.N, 256, c->P, c->S, h, with_q ? 2 : 0);
+		// (with the work queue, and where the heating terms are kept, the
+		// sub-cycles run in a pass of their own)
+		if (c->u_fixed && c->P.thermo_subcycling && !c->S.thq && !c->S.H) {
+			LAUNCH(KF(k_thermo_lean), c->P.N, 256, c->P, c->S, h, 0);
+		} else {
+			thermo_integrate(c, h);
+			if (c->u_fixed) LAUNCH(KF(k_thermo_lean), c->P.N, 256, c->P, c->S, h, 1);
+			else LAUNCH(KF(k_thermo_update_fp64), c->P.N, 256, c->P, c->S, h, with_q ? 2 : 0);
+		}
 		c->q_fresh = with_q;
 		break;
 	}
+	c->u_fixed = c->mixed;
 }
 
 void hydro_step(trg_ctx* c) {
@@ -715,6 +729,7 @@ void enqueue_full_step(trg_ctx* c, double dt_next) {
 		return;
 	}
 	// Torch::fullStep, Torch.cpp:389-418
+	c->u_fixed = c->mixed && c->q_fresh;  // the last sub-step's update left Q
 	if (!c->q_fresh) q_from_u(c, 0, 1);
 	c->q_fresh = false;
 	if (c->prologue_colden) {  // a slab's deferred prologue sweep (of this Q: no second sweep below)
