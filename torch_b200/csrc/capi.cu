@@ -677,6 +677,12 @@ void cons_record(trg_ctx* c, bool fused) {
 	}
 }
 
+// Threads of the time-step reduction: a cell each, at most 8 blocks per SM,
+// unless every 256 cells have a conservation partial (or, in a batch, a grid).
+long long dt_threads(const trg_ctx* c) {
+	return c->P.batch || c->S.cons_part ? c->P.N : std::min<long long>(c->P.N, 148LL * 8 * 256);
+}
+
 void time_step(trg_ctx* c, double dt_next) {
 	// Torch::calculateTimeStep and the min with dt_next_checkpoint (Torch.cpp:304-339, :394)
 	int step = c->steps < c->dt_hist_cap ? (int)c->steps : -1;
@@ -694,7 +700,7 @@ void time_step(trg_ctx* c, double dt_next) {
 	// the reduction's last block takes the step, unless the minima of the other
 	// slabs come in between
 	const DtEnd end{c->xfn ? 0 : 1, step, dt_next};
-	LAUNCH(KF(k_dt_reduce_fp64), c->P.N, 256, c->P, c->S, first_cell, end);
+	LAUNCH(KF(k_dt_reduce_fp64), dt_threads(c), 256, c->P, c->S, first_cell, end);
 	if (c->cons_on) cons_record(c, true);
 	if (end.on) return;
 	dt_exchange(c);
@@ -1248,7 +1254,7 @@ int trg_component(trg_ctx* c, int comp, int phase, double dt, double* out) {
 			first_cell = c->hs.first_nonwind_cell;
 			c->rad_once_pending = 0;
 		}
-		LAUNCH(KF(k_dt_reduce_fp64), c->P.N, 256, c->P, c->S, first_cell, (DtEnd{0, -1, 0.0}));
+		LAUNCH(KF(k_dt_reduce_fp64), dt_threads(c), 256, c->P, c->S, first_cell, (DtEnd{0, -1, 0.0}));
 		double mins[3];
 		CUDA_TRY(cudaMemcpyAsync(mins, c->S.scal + 2, sizeof(mins), cudaMemcpyDeviceToHost, c->stream));
 		CUDA_TRY(cudaStreamSynchronize(c->stream));

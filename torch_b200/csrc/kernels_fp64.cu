@@ -1078,7 +1078,14 @@ __device__ __forceinline__ void b_rad_heating_fp64(const Params& P, const State&
 	cell_ijk(P, id, ijk);
 	cell_xc(P, ijk, xc);
 	if (is_wind(P, id, ijk, xc)) return;
-	rad_heating_cell(P, S, id, FLD(S.Q, HII, id), FLD(S.Q, PRE, id), FLD(S.Q, DEN, id));
+	const double q_hii = FLD(S.Q, HII, id);
+	// neutral gas that no ionising photon reaches (exp(-TAU) = 0): every term is
+	// an exact 0 (only the diagnostics' 0/0 differs), known from 16 bytes
+	if (q_hii == 0 && !S.H && RFLD(S.R, R_TAU, id) >= 750.0) {
+		RFLD(S.R, R_HEAT, id) = 0;
+		return;
+	}
+	rad_heating_cell(P, S, id, q_hii, FLD(S.Q, PRE, id), FLD(S.Q, DEN, id));
 }
 __global__ void __launch_bounds__(256) k_rad_heating_fp64(Params P, State S) {
 	if (TRG_BATCHED && P.batch) {
@@ -1712,12 +1719,15 @@ __device__ __forceinline__ double block_min(double v) {
 // partial of the global FP64 mass and energy sums of the state (U), the
 // conservation check of the step.
 //
+// A block of a large grid takes many cells per thread, so that its three
+// block-wide minima, its atomics and its count are few.
+//
 // The last block of a grid to finish (end.on) also takes the time step from
 // the minima, so that no launch of its own follows (a slab's minima first go
 // through the exchange: end.on = 0 and k_dt_finalize).
 __device__ __forceinline__ void b_dt_finalize(const Params& P, const State& S, double dt_next, int first_time, int step);
-__device__ __forceinline__ void b_dt_reduce_fp64(const Params& P, const State& S, long long id, long long first_cell,
-                                                 double* cons_part);
+__device__ __forceinline__ void b_dt_reduce_fp64(const Params& P, const State& S, long long id, long long stride,
+                                                 long long first_cell, double* cons_part);
 __device__ __forceinline__ void dt_end(const Params& P, const State& S, const DtEnd& end, unsigned nblocks) {
 	if (!end.on || threadIdx.x != 0) return;
 	__threadfence();  // this block's minima before its count
@@ -1725,22 +1735,84 @@ __device__ __forceinline__ void dt_end(const Params& P, const State& S, const Dt
 	__threadfence();
 	b_dt_finalize(P, S, end.dt_next, 0, end.step);
 }
-__global__ void __launch_bounds__(256) k_dt_reduce_fp64(Params P, State S, long long first_cell, DtEnd end) {
+__global__ void __launch_bounds__(256, 4) k_dt_reduce_fp64(Params P, State S, long long first_cell, DtEnd end) {
 	if (TRG_BATCHED && P.batch) {
 		// grid ranges are padded to whole blocks: the block reduction stays within one grid
 		const BatchTable& B = *P.batch;
 		const int g = batch_slot(B.cell_off, B.G, blockIdx.x * (long long)blockDim.x);
 		const long long lid = blockIdx.x * (long long)blockDim.x + threadIdx.x - B.cell_off[g];
-		b_dt_reduce_fp64(B.P[g], B.S[g], lid, first_cell >= 0 ? B.first_cell[g] : -1, nullptr);
+		b_dt_reduce_fp64(B.P[g], B.S[g], lid, B.P[g].N, first_cell >= 0 ? B.first_cell[g] : -1, nullptr);
 		dt_end(B.P[g], B.S[g], end, (unsigned)((B.cell_off[g + 1] - B.cell_off[g]) / blockDim.x));
 		return;
 	}
-	b_dt_reduce_fp64(P, S, blockIdx.x * (long long)blockDim.x + threadIdx.x, first_cell, S.cons_part);
+	b_dt_reduce_fp64(P, S, blockIdx.x * (long long)blockDim.x + threadIdx.x, gridDim.x * (long long)blockDim.x,
+	                 first_cell, S.cons_part);
 	dt_end(P, S, end, gridDim.x);
 }
-__device__ __forceinline__ void b_dt_reduce_fp64(const Params& P, const State& S, long long id, long long first_cell,
-                                                 double* cons_part) {
-	double th = 1.0e308, tr = 1.0e308, tt = 1.0e308;
+// One cell's limits into the running ones: the largest 1/t of hydrodynamics
+// (its minimum time is half the reciprocal of that, rounded the same), the
+// least radiation and thermal times.
+struct DtMin {
+	double inv_t, rad, thermo;
+};
+__device__ __forceinline__ void dt_cell(const Params& P, const State& S, long long id, long long first_cell,
+                                        const double* inv_dx, DtMin& m) {
+	double q_den = FLD(S.Q, DEN, id), q_pre = FLD(S.Q, PRE, id), q_hii = FLD(S.Q, HII, id);
+	double inv_t = 0;
+	double ss = sqrt(P.gamma * q_pre / q_den);
+	#pragma unroll
+#ifdef TRG_FAST_MATH
+	for (int dim = 0; dim < 3; ++dim) if (dim < P.nd) inv_t += (fabs(FLD(S.Q, VEL + dim, id)) + ss) * inv_dx[dim];
+#else
+	for (int dim = 0; dim < 3; ++dim) if (dim < P.nd) inv_t += (fabs(FLD(S.Q, VEL + dim, id)) + ss) / P.dx[dim];
+#endif
+	if (inv_t == 0) inv_t = 1.0 / P.dt_max;
+	m.inv_t = smax(m.inv_t, inv_t);
+	int ijk[3];
+	double xc[3];
+	cell_ijk(P, id, ijk);
+	cell_xc(P, ijk, xc);
+	if (P.radiation_on && P.star_on && !is_wind(P, id, ijk, xc)) {
+		double dt_max = P.dt_max;
+		double dtc = dt_max, dt1 = dt_max, dt2 = dt_max, dt3 = dt_max, dt4 = dt_max;
+		if (P.coupling == CP_NEQ) {
+			double heat = RFLD(S.R, R_HEAT, id);
+			if (heat != 0) dtc = fabs(FLD(S.U, PRE, id) / heat);
+		}
+		if (P.K1 != 0.0) {
+			if (id == first_cell || q_hii != 0) {
+				const double rr = spline_eval(S.tables->rad_recomb, calc_temperature(P, q_hii, q_pre, q_den));
+				dt1 = P.K1 * P.hydrogenMass / (id == first_cell ? P.X * q_den * rr : P.X * q_den * q_hii * rr);
+			}
+		}
+		if (P.K3 != 0.0 || P.K4 != 0.0) {
+			double nH = P.X * q_den / P.hydrogenMass;
+			double nHI = (1.0 - q_hii) * nH;
+			double A_pi = photoionisation_rate(nHI, RFLD(S.R, R_TAU, id), RFLD(S.R, R_DTAU, id), S.shellVol[id], P.photonRate);
+			double Tq = calc_temperature(P, q_hii, q_pre, q_den);
+			double A_ci = collisional_ionisation_rate(P, Tq);
+			double A_rr = spline_eval(S.tables->rad_recomb, Tq);
+			double fracRate = (1.0 - q_hii) * (A_pi + q_hii * nH * A_ci) - q_hii * q_hii * nH * A_rr;
+			if (P.K3 != 0.0 && fracRate != 0.0) dt3 = P.K3 * smax(0.05, 1.0 - q_hii) / fabs(fracRate);
+			if (P.K4 != 0.0 && fracRate != 0.0) dt4 = P.K4 * 1.0 / fabs(fracRate);
+		}
+		const double tr = smin(dt_max, smin(dtc, smin(dt1, smin(dt2, smin(dt3, dt4)))));
+		if (tr == 0.0 || tr != tr || isinf(tr)) atomicOr(S.err, ERRB_DT);
+		m.rad = smin(m.rad, tr);
+	}
+	if (P.cooling_on) {
+		double rate = TFLD(S.T, T_RATE, id);
+		if (rate != 0) {
+			double frac = P.thermo_subcycling ? 1.0 : 0.1;
+			m.thermo = smin(m.thermo, fabs(frac * FLD(S.U, PRE, id) / rate));
+		}
+	}
+}
+// The block's cells: id, id + stride, ... below P.N (with cons_part, whose
+// partials belong to 256 cells each, id alone).
+__device__ __forceinline__ void b_dt_reduce_fp64(const Params& P, const State& S, long long id, long long stride,
+                                                 long long first_cell, double* cons_part) {
+	DtMin m = {0.0, 1.0e308, 1.0e308};
 	DD cm = {0.0, 0.0}, ce = {0.0, 0.0};
 	if (cons_part && id < P.N) {
 		int ijk[3];
@@ -1751,64 +1823,17 @@ __device__ __forceinline__ void b_dt_reduce_fp64(const Params& P, const State& S
 		cm = dd_prod(FLD(S.U, DEN, id), vol);
 		ce = dd_prod(FLD(S.U, PRE, id), vol);
 	}
-	if (id < P.N) {
-		double q_den = FLD(S.Q, DEN, id), q_pre = FLD(S.Q, PRE, id), q_hii = FLD(S.Q, HII, id);
-		double inv_t = 0;
-		double ss = sqrt(P.gamma * q_pre / q_den);
-		#pragma unroll
-#ifdef TRG_FAST_MATH
-		for (int dim = 0; dim < 3; ++dim) if (dim < P.nd) inv_t += (fabs(FLD(S.Q, VEL + dim, id)) + ss) * (1.0 / P.dx[dim]);
-#else
-		for (int dim = 0; dim < 3; ++dim) if (dim < P.nd) inv_t += (fabs(FLD(S.Q, VEL + dim, id)) + ss) / P.dx[dim];
-#endif
-		if (inv_t == 0) inv_t = 1.0 / P.dt_max;
-		th = 0.5 / inv_t;
-		int ijk[3];
-		double xc[3];
-		cell_ijk(P, id, ijk);
-		cell_xc(P, ijk, xc);
-		if (P.radiation_on && P.star_on && !is_wind(P, id, ijk, xc)) {
-			double dt_max = P.dt_max;
-			double dtc = dt_max, dt1 = dt_max, dt2 = dt_max, dt3 = dt_max, dt4 = dt_max;
-			if (P.coupling == CP_NEQ) {
-				double heat = RFLD(S.R, R_HEAT, id);
-				if (heat != 0) dtc = fabs(FLD(S.U, PRE, id) / heat);
-			}
-			if (P.K1 != 0.0) {
-				double T = calc_temperature(P, q_hii, q_pre, q_den);
-				if (id == first_cell)
-					dt1 = P.K1 * P.hydrogenMass / (P.X * q_den * spline_eval(S.tables->rad_recomb, T));
-				else if (q_hii != 0)
-					dt1 = P.K1 * P.hydrogenMass / (P.X * q_den * q_hii * spline_eval(S.tables->rad_recomb, T));
-			}
-			if (P.K3 != 0.0 || P.K4 != 0.0) {
-				double nH = P.X * q_den / P.hydrogenMass;
-				double nHI = (1.0 - q_hii) * nH;
-				double A_pi = photoionisation_rate(nHI, RFLD(S.R, R_TAU, id), RFLD(S.R, R_DTAU, id), S.shellVol[id], P.photonRate);
-				double Tq = calc_temperature(P, q_hii, q_pre, q_den);
-				double A_ci = collisional_ionisation_rate(P, Tq);
-				double A_rr = spline_eval(S.tables->rad_recomb, Tq);
-				double fracRate = (1.0 - q_hii) * (A_pi + q_hii * nH * A_ci) - q_hii * q_hii * nH * A_rr;
-				if (P.K3 != 0.0 && fracRate != 0.0) dt3 = P.K3 * smax(0.05, 1.0 - q_hii) / fabs(fracRate);
-				if (P.K4 != 0.0 && fracRate != 0.0) dt4 = P.K4 * 1.0 / fabs(fracRate);
-			}
-			tr = smin(dt_max, smin(dtc, smin(dt1, smin(dt2, smin(dt3, dt4)))));
-			if (tr == 0.0 || tr != tr || isinf(tr)) atomicOr(S.err, ERRB_DT);
-		}
-		if (P.cooling_on) {
-			double rate = TFLD(S.T, T_RATE, id);
-			if (rate != 0) {
-				double frac = P.thermo_subcycling ? 1.0 : 0.1;
-				tt = fabs(frac * FLD(S.U, PRE, id) / rate);
-			}
-		}
-	}
+	double inv_dx[3];
+#pragma unroll
+	for (int dim = 0; dim < 3; ++dim) inv_dx[dim] = dim < P.nd ? 1.0 / P.dx[dim] : 0.0;
+#pragma unroll 1
+	for (; id < P.N; id += stride) dt_cell(P, S, id, first_cell, inv_dx, m);
 	if (cons_part) block_cons_partial(cm, ce, cons_part, blockIdx.x);
-	th = block_min(th);
+	double th = block_min(m.inv_t > 0 ? 0.5 / m.inv_t : 1.0e308);
 	__syncthreads();
-	tr = block_min(tr);
+	double tr = block_min(m.rad);
 	__syncthreads();
-	tt = block_min(tt);
+	double tt = block_min(m.thermo);
 	if (threadIdx.x == 0) {
 		unsigned long long* slots = reinterpret_cast<unsigned long long*>(S.scal + 2);
 		atomicMin(&slots[0], dbits(th));

@@ -122,7 +122,10 @@ __device__ __forceinline__ double face_area(const Params& P, const double* xc, i
 }
 
 // Fluid::initialiseGrid wind test, Fluid.cpp:41-53.
+// Without a wind (radius 0) the distance vanishes in the star's own cell only:
+// its terms (i - s)(i + 1/2 - s) are 0 there and positive elsewhere.
 __device__ __forceinline__ bool is_wind(const Params& P, long long id, const int* ijk, const double* xc) {
+	if (P.wind_radius == 0) return id == P.star_cell;
 	double dist2 = 0;
 	#pragma unroll
 	for (int i = 0; i < 3; ++i) if (i < P.nd)
