@@ -832,8 +832,9 @@ int check_device_error(trg_ctx* c) {
 // 55), and beyond it for the column densities, whose cells take little
 // arithmetic (400 x 520: 0.61 against 1.74 ms).
 constexpr long long CHAIN_MAX_SHELL_RAD = 1024, CHAIN_MAX_SHELL_COL = 2048;
-int build_chain(trg_ctx* c, const std::vector<long long>& off, const int* d_cells, double inner_dist2,
-                long long most, const SweepChain** out, trg_ctx::ChainShape* shape) {
+int build_chain(trg_ctx* c, const std::vector<long long>& off, const int* d_cells, bool rad,
+                const SweepChain** out, trg_ctx::ChainShape* shape) {
+	const long long most = rad ? CHAIN_MAX_SHELL_RAD : CHAIN_MAX_SHELL_COL;
 	long long maxshell = 0;
 	for (size_t s = 0; s + 1 < off.size(); ++s) maxshell = std::max(maxshell, off[s + 1] - off[s]);
 	if (maxshell == 0 || maxshell > most || !c->shell_overlap) return TRG_OK;
@@ -862,7 +863,7 @@ int build_chain(trg_ctx* c, const std::vector<long long>& off, const int* d_cell
 	int* pos = reinterpret_cast<int*>(c->S.UDOT);  // zero between uses
 	CUDA_TRY(cudaMemsetAsync(pos, 0xff, c->P.N * sizeof(int), c->stream));
 	LAUNCH(KF(k_chain_positions), ch.n, 256, d_cells, ch.n, pos);
-	LAUNCH(KF(k_chain_tables), ch.n, 256, c->P, ch, pos, inner_dist2, slot, w, bad);
+	LAUNCH(KF(k_chain_tables), ch.n, 256, c->P, ch, pos, rad ? 1 : 0, slot, w, bad);
 	CUDA_TRY(cudaMemsetAsync(pos, 0, c->P.N * sizeof(int), c->stream));
 	int h_bad = 0;
 	CUDA_TRY(cudaMemcpyAsync(&h_bad, bad, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
@@ -1061,13 +1062,9 @@ int create_impl(const trg_params* p, const SlabSpec* slab, const double* den, co
 		else if (!std::strcmp(kb, "fast")) c->fastk = 1;
 	}
 	if (c->P.star_on && c->P.lbc[0] != BC_PARTITION && c->P.rbc[0] != BC_PARTITION) {
-		// (the distances within which a cell has no upwind neighbours are those
-		// of rad_shell and b_colden_shell_fp64)
 		if ((c->P.rt_scheme == 0 &&
-		     (rc = build_chain(c, c->hs.off_nonwind, c->d_sweep_nonwind, 0.95, CHAIN_MAX_SHELL_RAD, &S.chain_rad,
-		                       &c->chain_rad))) ||
-		    (rc = build_chain(c, c->hs.off_all, c->d_sweep_all, 0.95 * 0.95, CHAIN_MAX_SHELL_COL, &S.chain_col,
-		                       &c->chain_col)))
+		     (rc = build_chain(c, c->hs.off_nonwind, c->d_sweep_nonwind, true, &S.chain_rad, &c->chain_rad))) ||
+		    (rc = build_chain(c, c->hs.off_all, c->d_sweep_all, false, &S.chain_col, &c->chain_col)))
 			return rc;
 	}
 	// Torch::run prologue (Torch.cpp:245-264): Q from U with floors, and the

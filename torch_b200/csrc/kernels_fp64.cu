@@ -277,7 +277,31 @@ __device__ __forceinline__ void doric(double dt, double& HII_avg, double& HII, d
 	}
 }
 
-__device__ __forceinline__ double pick3(double a0, double a1, double a2, int k) { return k == 0 ? a0 : (k == 1 ? a1 : a2); }
+__device__ __forceinline__ int pick3(int a0, int a1, int a2, int k) { return k == 0 ? a0 : (k == 1 ? a1 : a2); }
+
+// A swept cell's index coordinates and its offset from the star in half cells,
+// e = 2 (xc - sxc): whole numbers, since cell centres and the star lie on
+// multiples of half a cell, so that every test of the sweeps' geometry is one
+// of integers (a third of the shell kernels' instructions when they were of
+// doubles).  The cell has upwind neighbours ("inner") unless it is the star's
+// or touches it: the reference's dist2 > 0.95 (Radiation.cpp:354) and > 0.95^2
+// (Thermodynamics.cpp:342) both mean that some |e| >= 2, as e^2 summed is 3 at
+// most otherwise.
+struct SweepCell {
+	int x[3];  // x global
+	int e[3];
+	__device__ __forceinline__ SweepCell(const Params& P, long long id) {
+		cell_ijk(P, id, x);
+		x[0] += P.x0;
+#pragma unroll
+		for (int i = 0; i < 3; ++i) e[i] = i < P.nd ? 2 * x[i] + 1 - P.star2[i] : 0;
+	}
+	__device__ __forceinline__ bool inner() const { return max(abs(e[0]), max(abs(e[1]), abs(e[2]))) >= 2; }
+	// Radiation::isStar (Radiation.cpp:682-684): z compares an int with a double
+	__device__ __forceinline__ bool star(const Params& P) const {
+		return x[0] == (int)P.sxc[0] && x[1] == (int)P.sxc[1] && 2 * x[2] == P.star2[2];
+	}
+};
 
 // C2-Ray upwind neighbours and weights (Grid::calculateNearestNeighbours,
 // Grid.cpp:922-952) computed on the fly.  A neighbour outside the interior
@@ -290,53 +314,54 @@ __device__ __forceinline__ double pick3(double a0, double a1, double a2, int k) 
 // its index into S.sweep_recv.
 // The rotated frame (irot) is resolved with selects rather than indexed
 // arrays, so that everything stays in registers.
-__device__ __forceinline__ void neighbours(const Params& P, const int* ijk, const double* xc, long long* nb, double* w) {
-	int plane = 0;
-	double dmax = 0;
-#pragma unroll
-	for (int i = 0; i < 3; ++i)
-		if (i < P.nd) {
-			double dd = fabs(xc[i] - P.sxc[i]);
-			if (dd > dmax) { dmax = dd; plane = i; }
-		}
+__device__ __forceinline__ void neighbours(const Params& P, const SweepCell& c, long long id, long long* nb, double* w) {
+	const int a0 = abs(c.e[0]), a1 = abs(c.e[1]), a2 = abs(c.e[2]);
+	int plane = a1 > a0 ? 1 : 0;
+	plane = a2 > max(a0, a1) ? 2 : plane;
 	// irot = {(plane + 1) % 3, (plane + 2) % 3, plane}
 	const int r0 = plane == 2 ? 0 : plane + 1, r1 = plane == 0 ? 2 : plane - 1, r2 = plane;
-	const double x0 = pick3(xc[0], xc[1], xc[2], r0), x1 = pick3(xc[0], xc[1], xc[2], r1);
-	const double d0 = x0 - pick3(P.sxc[0], P.sxc[1], P.sxc[2], r0);
-	const double d1 = x1 - pick3(P.sxc[0], P.sxc[1], P.sxc[2], r1);
-	const double d2 = pick3(xc[0], xc[1], xc[2], r2) - pick3(P.sxc[0], P.sxc[1], P.sxc[2], r2);
-	const int s0 = d0 < -1.0 / 10.0 ? -1 : 1, s1 = d1 < -1.0 / 10.0 ? -1 : 1, s2 = d2 < -1.0 / 10.0 ? -1 : 1;
-	const int L0 = fabs(d0) < 1.0 / 10.0 ? 0 : s0, L1 = fabs(d1) < 1.0 / 10.0 ? 0 : s1, L2 = fabs(d2) < 1.0 / 10.0 ? 0 : s2;
+	const int e0 = pick3(c.e[0], c.e[1], c.e[2], r0), e1 = pick3(c.e[0], c.e[1], c.e[2], r1);
+	const int e2 = pick3(c.e[0], c.e[1], c.e[2], r2);
+	const int s0 = e0 < 0 ? -1 : 1, s1 = e1 < 0 ? -1 : 1, s2 = e2 < 0 ? -1 : 1;
+	const int L0 = e0 == 0 ? 0 : s0, L1 = e1 == 0 ? 0 : s1, L2 = e2 == 0 ? 0 : s2;
 	// offsets in the rotated frame: n = 0: (0, 0, -L2), 1: (0, -L1, -L2), 2: (-L0, 0, -L2), 3: (-L0, -L1, -L2)
+	const int nxy = P.nx * P.ny, i = c.x[0] - P.x0;
+	const int o0 = L0 * pick3(1, P.nx, nxy, r0), o1 = L1 * pick3(1, P.nx, nxy, r1), o2 = L2 * pick3(1, P.nx, nxy, r2);
+	const int c0 = pick3(i, c.x[1], c.x[2], r0) - L0, c1 = pick3(i, c.x[1], c.x[2], r1) - L1;
+	const int c2 = pick3(i, c.x[1], c.x[2], r2) - L2;
+	const bool in0 = (unsigned)c0 < (unsigned)pick3(P.nx, P.ny, P.nz, r0);
+	const bool in1 = (unsigned)c1 < (unsigned)pick3(P.nx, P.ny, P.nz, r1);
+	const bool in2 = (unsigned)c2 < (unsigned)pick3(P.nx, P.ny, P.nz, r2);
 	const bool slab = P.lbc[0] == BC_PARTITION || P.rbc[0] == BC_PARTITION;  // the same for every thread
 #pragma unroll
 	for (int n = 0; n < 4; ++n) {
-		const int o0 = (n & 2) ? -L0 : 0, o1 = (n & 1) ? -L1 : 0, o2 = -L2;
-		const int ti = ijk[0] + (r0 == 0 ? o0 : 0) + (r1 == 0 ? o1 : 0) + (r2 == 0 ? o2 : 0);
-		const int tj = ijk[1] + (r0 == 1 ? o0 : 0) + (r1 == 1 ? o1 : 0) + (r2 == 1 ? o2 : 0);
-		const int tk = ijk[2] + (r0 == 2 ? o0 : 0) + (r1 == 2 ? o1 : 0) + (r2 == 2 ? o2 : 0);
-		const bool yz = tj >= 0 && tj < P.ny && tk >= 0 && tk < P.nz;
-		const bool in = ti >= 0 && ti < P.nx && yz;
-		nb[n] = in ? flat_id(P, ti, tj, tk) : -1;
-		if (slab && !in && yz &&
-		    ((ti == -1 && P.lbc[0] == BC_PARTITION) || (ti == P.nx && P.rbc[0] == BC_PARTITION)))
-			nb[n] = -2 - ((ti < 0 ? 0 : (long long)P.ny * P.nz) + tj + (long long)P.ny * tk);
+		const bool in = in2 && (in0 || !(n & 2)) && (in1 || !(n & 1));
+		nb[n] = in ? id - o2 - ((n & 2) ? o0 : 0) - ((n & 1) ? o1 : 0) : -1;
+		if (slab && !in) {
+			const int m0 = (n & 2) ? L0 : 0, m1 = (n & 1) ? L1 : 0;
+			const int ti = i - (r0 == 0 ? m0 : 0) - (r1 == 0 ? m1 : 0) - (r2 == 0 ? L2 : 0);
+			const int tj = c.x[1] - (r0 == 1 ? m0 : 0) - (r1 == 1 ? m1 : 0) - (r2 == 1 ? L2 : 0);
+			const int tk = c.x[2] - (r0 == 2 ? m0 : 0) - (r1 == 2 ? m1 : 0) - (r2 == 2 ? L2 : 0);
+			if (tj >= 0 && tj < P.ny && tk >= 0 && tk < P.nz &&
+			    ((ti == -1 && P.lbc[0] == BC_PARTITION) || (ti == P.nx && P.rbc[0] == BC_PARTITION)))
+				nb[n] = -2 - ((ti < 0 ? 0 : (long long)P.ny * P.nz) + tj + (long long)P.ny * tk);
+		}
 	}
-	double ic0 = (int)x0 - 0.5 * (s2 * d0 / d2);
-	double ic1 = (int)x1 - 0.5 * (s2 * d1 / d2);
-	double delta0 = fabs(2.0 * ic0 - 2.0 * (int)x0 + s0);
-	double delta1 = fabs(2.0 * ic1 - 2.0 * (int)x1 + s1);
-	w[0] = (fabs(d2) > 0.9) ? delta0 * delta1 : 0;
-	w[1] = ((fabs(d1) > 0.9) && (fabs(d2) > 0.9)) ? delta0 * (1.0 - delta1) : 0;
-	w[2] = ((fabs(d0) > 0.9) && (fabs(d2) > 0.9)) ? (1.0 - delta0) * delta1 : 0;
-	w[3] = ((fabs(d0) > 0.9) && (fabs(d1) > 0.9) && (fabs(d2) > 0.9)) ? (1.0 - delta0) * (1.0 - delta1) : 0;
-}
-
-__device__ __forceinline__ double dist2_cells(const Params& P, const double* xc) {
-	double d2 = 0;
-	#pragma unroll
-	for (int i = 0; i < 3; ++i) if (i < P.nd) d2 += (xc[i] - P.sxc[i]) * (xc[i] - P.sxc[i]);
-	return d2;
+	const double x0 = pick3(c.x[0], c.x[1], c.x[2], r0), x1 = pick3(c.x[0], c.x[1], c.x[2], r1);
+#ifdef TRG_FAST_MATH
+	const double inv2 = (double)s2 / (double)e2;
+	const double ic0 = x0 - 0.5 * ((double)e0 * inv2), ic1 = x1 - 0.5 * ((double)e1 * inv2);
+#else
+	const double ic0 = x0 - 0.5 * ((double)(s2 * e0) / (double)e2);
+	const double ic1 = x1 - 0.5 * ((double)(s2 * e1) / (double)e2);
+#endif
+	const double delta0 = fabs(2.0 * ic0 - 2.0 * x0 + s0);
+	const double delta1 = fabs(2.0 * ic1 - 2.0 * x1 + s1);
+	const bool far0 = abs(e0) >= 2, far1 = abs(e1) >= 2, far2 = abs(e2) >= 2;  // |d| > 0.9
+	w[0] = far2 ? delta0 * delta1 : 0;
+	w[1] = far1 && far2 ? delta0 * (1.0 - delta1) : 0;
+	w[2] = far0 && far2 ? (1.0 - delta0) * delta1 : 0;
+	w[3] = far0 && far1 && far2 ? (1.0 - delta0) * (1.0 - delta1) : 0;
 }
 
 // Programmatic dependent launch.  The shells of a sweep after the first are
@@ -541,14 +566,10 @@ __device__ __forceinline__ void rad_shell(const Params& P, const State& S, const
 	long long nb[4] = {-1, -1, -1, -1};
 	double w[4] = {0, 0, 0, 0};
 	// everything that does not depend on the inner shells
-	int ijk[3];
-	double xc[3];
-	cell_ijk(P, id, ijk);
-	cell_xc(P, ijk, xc);
-	inner = dist2_cells(P, xc) > 0.95;
-	if (inner) neighbours(P, ijk, xc, nb, w);
-	// Radiation::isStar (Radiation.cpp:682-684): z compares an int with a double.
-	star = (int)xc[0] == (int)P.sxc[0] && (int)xc[1] == (int)P.sxc[1] && (double)(int)xc[2] == P.sxc[2];
+	const SweepCell cell(P, id);
+	inner = cell.inner();
+	if (inner) neighbours(P, cell, id, nb, w);
+	star = cell.star(P);
 	if (SW) {
 		nH_cell = sw[0];
 		q_hii = sw[3 * swn];
@@ -944,14 +965,11 @@ __global__ void __launch_bounds__(256) k_batch_learned_prep(Params Pv, State Sv)
 // shell per launch); the fractions are then updated by one launch over all
 // non-wind cells, which are independent of each other in these schemes.
 __device__ __forceinline__ void b_rad_tau_shell(const Params& P, const State& S, long long id) {
-	int ijk[3];
-	double xc[3];
-	cell_ijk(P, id, ijk);
-	cell_xc(P, ijk, xc);
-	const bool inner = dist2_cells(P, xc) > 0.95;
+	const SweepCell cell(P, id);
+	const bool inner = cell.inner();
 	long long nb[4];
 	double w[4];
-	if (inner) neighbours(P, ijk, xc, nb, w);
+	if (inner) neighbours(P, cell, id, nb, w);
 	const double nH = P.X * FLD(S.Q, DEN, id) / P.hydrogenMass;
 	const double dtau = (1.0 - FLD(S.Q, HII, id)) * nH * P.photoIonXsec * S.ds[id];
 	const double dtau_a = (1.0 - RFLD(S.R, R_HII_A, id)) * nH * P.photoIonXsec * S.ds[id];
@@ -977,12 +995,8 @@ __global__ void __launch_bounds__(128) k_rad_tau_shell(Params P, State S, const 
 // iteration with tau_avg = TAU) and explicit (one doric step whose
 // time-averaged result becomes Q[HII]; HII_A is not written).
 __device__ __forceinline__ void b_rad_solve2(const Params& P, const State& S, long long id, double h) {
-	int ijk[3];
-	double xc[3];
-	cell_ijk(P, id, ijk);
-	cell_xc(P, ijk, xc);
 	const double dt = h * S.scal[0];
-	if ((int)xc[0] == (int)P.sxc[0] && (int)xc[1] == (int)P.sxc[1] && (double)(int)xc[2] == P.sxc[2]) {
+	if (SweepCell(P, id).star(P)) {
 		RFLD(S.R, R_HEAT, id) = 0;
 		FLD(S.Q, HII, id) = 1;
 		RFLD(S.R, R_HII_A, id) = 1;
@@ -1287,14 +1301,11 @@ __device__ __forceinline__ double colden_interp(const double* colden, const doub
 // `own`: the cell's ds rho / m_H in the sweep-ordered array, or null.
 __device__ __forceinline__ void b_colden_shell_fp64(const Params& P, const State& S, long long id,
                                                     const double* own = nullptr) {
-	int ijk[3];
-	double xc[3];
-	cell_ijk(P, id, ijk);
-	cell_xc(P, ijk, xc);
-	const bool inner = dist2_cells(P, xc) > 0.95 * 0.95;
+	const SweepCell cell(P, id);
+	const bool inner = cell.inner();
 	long long nb[4];
 	double w0[4];
-	if (inner) neighbours(P, ijk, xc, nb, w0);
+	if (inner) neighbours(P, cell, id, nb, w0);
 	const double dcolden = own ? *own : (FLD(S.Q, DEN, id) / P.hydrogenMass) * S.ds[id];
 	const double2* src[4] = {nullptr, nullptr, nullptr, nullptr};
 	if (inner) nb_sources<2>(S, S.T, nb, w0, src);

@@ -322,6 +322,9 @@ std::string host_setup(const trg_params& p, const double* den, const double* pre
 	}
 	if (P.nd < 3) P.sxc[2] = 0;
 	if (P.nd < 2) P.sxc[1] = 0;
+	for (int i = 0; i < 3; ++i) P.star2[i] = (int)(2.0 * P.sxc[i]);
+	P.div_nx = make_div_by((unsigned)P.nx);
+	P.div_ny = make_div_by((unsigned)P.ny);
 	Geo g(P);
 	// the star's cell in this grid's (a slab's) own indices
 	const int sp_loc[3] = {p.star_pos[0] - P.x0, p.star_pos[1], p.star_pos[2]};

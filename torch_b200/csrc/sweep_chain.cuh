@@ -371,18 +371,17 @@ __device__ __forceinline__ int shell_at(const SweepChain& ch, int p) {
 	return lo;
 }
 __global__ void __launch_bounds__(256) k_chain_tables(Params P, SweepChain ch, const int* __restrict__ pos,
-                                                      double inner_dist2, ChainSlots* __restrict__ slot,
+                                                      int rad, ChainSlots* __restrict__ slot,
                                                       double* __restrict__ w, int* __restrict__ bad) {
 	const int t = blockIdx.x * blockDim.x + threadIdx.x;
 	if (t >= ch.n) return;
 	const int s = shell_at(ch, t);
-	int ijk[3], code[4] = {-1, -1, -1, -1};
-	double xc[3], w0[4] = {1.0, 0.0, 0.0, 0.0};
-	cell_ijk(P, ch.cells[t], ijk);
-	cell_xc(P, ijk, xc);
-	if (dist2_cells(P, xc) > inner_dist2) {
+	int code[4] = {-1, -1, -1, -1};
+	double w0[4] = {1.0, 0.0, 0.0, 0.0};
+	const SweepCell cell(P, ch.cells[t]);
+	if (cell.inner()) {
 		long long nb[4];
-		neighbours(P, ijk, xc, nb, w0);
+		neighbours(P, cell, ch.cells[t], nb, w0);
 #pragma unroll
 		for (int k = 0; k < 4; ++k) {
 			if (w0[k] == 0 || nb[k] < 0 || pos[nb[k]] < 0) continue;
@@ -391,8 +390,7 @@ __global__ void __launch_bounds__(256) k_chain_tables(Params P, SweepChain ch, c
 			code[k] = (sn % 3) * ch.maxshell + (p - ch.off[sn]);
 		}
 	}
-	if ((int)xc[0] == (int)P.sxc[0] && (int)xc[1] == (int)P.sxc[1] && (double)(int)xc[2] == P.sxc[2] && inner_dist2 > 0.94)
-		*bad = 1;  // a swept star cell (Radiation::isStar) is not solved: left to the per-shell kernels
+	if (rad && cell.star(P)) *bad = 1;  // a swept star cell (Radiation::isStar) is not solved: left to the per-shell kernels
 	slot[t] = ChainSlots{code[0], code[1], code[2], code[3]};
 #pragma unroll
 	for (int k = 0; k < 4; ++k) w[(long long)k * ch.n + t] = w0[k];

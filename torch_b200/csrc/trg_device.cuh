@@ -41,12 +41,11 @@ __device__ __forceinline__ double smin(double a, double b) { return (b < a) ? b 
 __device__ __forceinline__ double smax(double a, double b) { return (a < b) ? b : a; }
 
 __device__ __forceinline__ void cell_ijk(const Params& P, long long id, int* ijk) {
-	if (P.N <= 0x7fffffffLL) {  // 32-bit division: a fraction of the cost of the 64-bit one
-		unsigned u = (unsigned)id, nx = (unsigned)P.nx, ny = (unsigned)P.ny;
-		unsigned q = u / nx;
-		ijk[0] = (int)(u - q * nx);
-		unsigned r = q / ny;
-		ijk[1] = (int)(q - r * ny);
+	if (P.N <= 0x7fffffffLL) {  // two multiplications instead of the 64-bit divisions
+		const unsigned u = (unsigned)id;
+		const unsigned q = div_by(u, P.div_nx), r = div_by(q, P.div_ny);
+		ijk[0] = (int)(u - q * (unsigned)P.nx);
+		ijk[1] = (int)(q - r * (unsigned)P.ny);
 		ijk[2] = (int)r;
 		return;
 	}

@@ -26,7 +26,7 @@
 	__global__ void k_rad_chain(Params P, State S, double h); \
 	__global__ void k_colden_chain(Params P, State S); \
 	__global__ void k_chain_positions(const int* cells, int n, int* pos); \
-	__global__ void k_chain_tables(Params P, SweepChain ch, const int* pos, double inner_dist2, ChainSlots* slot, \
+	__global__ void k_chain_tables(Params P, SweepChain ch, const int* pos, int rad, ChainSlots* slot, \
 	                               double* w, int* bad); \
 	__global__ void k_rad_no_star_fp64(Params P, State S, double h); \
 	__global__ void k_rad_tau_shell(Params P, State S, const int* cells, int count); \

@@ -94,6 +94,22 @@ struct SweepChain {
 };
 constexpr int CHAIN_GROUP = 256;  // most threads of one of the two groups that take a chain's shells in turn
 
+// Division of a non-negative 31-bit index by a fixed divisor: n / d =
+// (n m) >> s with s = 31 + ceil(log2 d) and m = ceil(2^s / d) <= 2^32 - 1 or
+// 2^31 (T. Granlund and P. Montgomery, "Division by invariant integers using
+// multiplication", PLDI 1994): m d exceeds 2^s by less than 2^(s - 31), so the
+// product's error stays below 2^s.
+struct DivBy {
+	unsigned m, s;
+};
+inline DivBy make_div_by(unsigned d) {
+	unsigned l = 0;
+	while ((1ull << l) < d) ++l;
+	const unsigned s = 31 + l;
+	return DivBy{(unsigned)(((1ull << s) + d - 1) / d), s};
+}
+TRG_HD inline unsigned div_by(unsigned n, const DivBy& d) { return (unsigned)(((unsigned long long)n * d.m) >> d.s); }
+
 struct Params {
 	int nd, nx, ny, nz;
 	long long N;
@@ -117,6 +133,8 @@ struct Params {
 	int wind_radius;     // Star::windCellRadius when the star is on, else 0
 	long long star_cell; // flat index of the star cell or -1
 	double sxc[3];       // Star::xc
+	int star2[3];        // twice Star::xc, whole numbers (0 beyond nd)
+	DivBy div_nx, div_ny;
 	double mdot, edot;
 	// thermodynamics constants (Thermodynamics::initialise, Thermodynamics.cpp:24-57)
 	double z0, T1, T2, T3, T4, imlc, nmlc, ciec_minT, ciec, cxhi_damp, n0, nmc;
