@@ -539,6 +539,8 @@ __device__ __forceinline__ double inv_logit10(float l) {
 	return 1.0 / (1.0 + exp10(-v));
 }
 
+#include "rad_solve.cuh"
+
 // One shell of the causal sweep of Radiation::transferRadiation
 // (Radiation.cpp:600-612): tau interpolation, the implicit HII update
 // (update_HIIfrac, :375-478) and the new optical depths.  Every cell of a
@@ -897,13 +899,65 @@ __device__ __forceinline__ void b_rad_sweep_prep(const Params& P, const State& S
 		}
 	}
 }
+// The plain solve of a shell's cell (no learned start, counters or recording)
+// from its sweep-ordered inputs: rad_shell<false, true> with the solver of
+// rad_solve.cuh, whose first exponential and reciprocals are formed before the
+// wait for the previous shell.  In the exact build, where a cell's divisions
+// and exponentials are the shell's time: 100^3 HII region 372 -> 261 us per sweep.
+// The fast build keeps the general loop: its large shells are bound by FP64
+// issue, of which these reciprocals take more (256^3: 1.44 -> 1.49-1.58 ms).
+__device__ __forceinline__ void rad_shell_plain(const Params& P, const State& S, long long id, double h, double* sw,
+                                                long long swn) {
+	const double dt = h * S.scal[0];
+	SolveCell c;
+	c.n_H = sw[0];
+	c.alphaB = sw[swn];
+	c.A_ci = sw[2 * swn];
+	c.x = sw[3 * swn];
+	c.ds = sw[4 * swn];
+	c.shellVol = sw[5 * swn];
+	const SweepCell cell(P, id);
+	const bool inner = cell.inner(), star = cell.star(P);
+	long long nb[4] = {-1, -1, -1, -1};
+	double w[4] = {1.0, 0.0, 0.0, 0.0};
+	if (inner) neighbours(P, cell, id, nb, w);
+	const double2* src[4];
+	nb_sources<4>(S, S.R, nb, w, src);
+	solve_pre(P, c);
+	sweep_wait();
+	double a[4] = {0, 0, 0, 0}, b[4] = {0, 0, 0, 0}, tau, tau_a;
+#pragma unroll
+	for (int i = 0; i < 4; ++i)
+		if (src[i]) {
+			const double2 u = __ldcg(src[i]), v = __ldcg(src[i] + 1);
+			a[i] = u.x + u.y;
+			b[i] = v.x + v.y;
+		}
+	tau_interp2(P, a, b, w, tau, tau_a);
+	sw[SW_TAU_A * swn] = tau_a;  // the next sweep's learned-start candidates are chosen from it
+	double x_new = 1, x_avg = 1;
+	if (star) {
+		RFLD(S.R, R_HEAT, id) = 0;
+	} else {
+		solve_cell(P, S, c, dt, tau_a, x_new, x_avg);
+		if (x_new > 0.001) FLD(S.Q, ADV, id) = 1;
+	}
+	RFLD(S.R, R_HII_A, id) = x_avg;
+	FLD(S.Q, HII, id) = x_new;
+	store_taus(S, id, tau, (1.0 - x_new) * c.n_H * P.photoIonXsec * c.ds, tau_a,
+	           (1.0 - x_avg) * c.n_H * P.photoIonXsec * c.ds);
+}
 // A radiation shell reading its cells' own inputs from S.sw_rad; `off` is the
 // shell's offset in the non-wind sweep list.
 __global__ void TRG_RAD_SHELL_BOUNDS k_rad_shell_sw(Params P, State S, const int* __restrict__ cells, int count,
                                                      double h, long long off) {
 	const int t = blockIdx.x * blockDim.x + threadIdx.x;
 	if (t >= count) return;
+#ifdef TRG_FAST_MATH
 	rad_shell<false, true>(P, S, cells[t], h, S.sw_rad + off + t, S.sw_rad_n);
+#else
+	rad_shell_plain(P, S, cells[t], h, S.sw_rad + off + t, S.sw_rad_n);
+#endif
 }
 // The same with the solver counters and training-set recording compiled in.
 __global__ void __launch_bounds__(128) k_rad_shell_sw_diag(Params P, State S, const int* __restrict__ cells,
@@ -1297,6 +1351,33 @@ __device__ __forceinline__ double colden_interp(const double* colden, const doub
 	return newcolden;
 }
 
+// The same with its divisions overlapped (Recip); the fast build has one only.
+__device__ __forceinline__ double colden_interp_recip(const double* c, const double* w0) {
+#ifdef TRG_FAST_MATH
+	return colden_interp(c, w0);
+#else
+	double w[4], sum = 0.0, out = 0.0;
+	bool ok = true;
+#pragma unroll
+	for (int i = 0; i < 4; ++i) {
+		Recip r;
+		r.set(c[i] == 0 ? 1.0 : c[i]);
+		const double n = c[i] == 0 ? 0.0 : w0[i];
+		ok &= r.takes(n);
+		w[i] = r.quotient(n);
+	}
+	sum = w[0] + w[1] + w[2] + w[3];
+	Recip rs;
+	rs.set(sum);
+#pragma unroll
+	for (int i = 0; i < 4; ++i) {
+		ok &= rs.takes(w[i]);
+		out += rs.quotient(w[i]) * c[i];
+	}
+	return ok ? out : colden_interp(c, w0);  // (a zero sum is not taken)
+#endif
+}
+
 // One shell of Thermodynamics::rayTrace / updateColDen (Thermodynamics.cpp:339-417).
 // `own`: the cell's ds rho / m_H in the sweep-ordered array, or null.
 __device__ __forceinline__ void b_colden_shell_fp64(const Params& P, const State& S, long long id,
@@ -1318,7 +1399,7 @@ __device__ __forceinline__ void b_colden_shell_fp64(const Params& P, const State
 				const double2 c = __ldcg(src[i]);  // COL_DEN, DCOL_DEN
 				colden[i] = c.x + c.y;
 			}
-		newcolden = colden_interp(colden, w0);
+		newcolden = colden_interp_recip(colden, w0);
 	}
 	reinterpret_cast<double2*>(S.T + id * 2)[0] = make_double2(newcolden, dcolden);
 }
