@@ -12,7 +12,7 @@ import pytest
 import common  # noqa: F401  (paths)
 import known_answers
 import torch_b200
-from torch_b200 import workloads
+from torch_b200 import config, workloads
 
 pytestmark = pytest.mark.gpu
 
@@ -86,3 +86,30 @@ def test_batched_chains_equal_single_grids(sizes):
         t.close()
         for f in ("U", "Q", "R", "T"):
             assert np.array_equal(getattr(s, f), getattr(ref, f)), f
+
+
+@pytest.mark.parametrize("form", [torch_b200.PRECISION_FP64, torch_b200.PRECISION_FP32])
+def test_tied_axes_read_no_cell_of_their_own_shell(monkeypatch, form):
+    """A star in a cell's centre: on the diagonals two axes tie, and a neighbour
+    level with the cell belongs to the cell's own shell.  Its weight is exactly
+    0 in both builds (49 times the rounded 1/49 is not 1), or the chain would be
+    refused and the sweeps launched shell by shell (two times 65 launches)."""
+    n = 131
+    tp = workloads.hii_region_parameters(n=n)
+    tp = dataclasses.replace(tp, nd=2, ncells=(n, n, 1), star_position=(65, 65, 0))
+    rng = np.random.default_rng(2)
+    den = 1e3 * workloads.setups.HYDROGEN_MASS * np.exp(0.3 * rng.standard_normal(n * n))
+    ic = config.make_initial_conditions((n, n, 1), tp.sideLength / n, den,
+                                        den * workloads.setups.SPECIFIC_GAS_CONSTANT * 100.0, np.zeros(n * n),
+                                        np.zeros((3, n * n)))
+    t = torch_b200.Torch(tp, ic, precision=form)
+    before = t.kernel_launches()
+    t.run_steps(6)
+    launches = t.kernel_launches() - before
+    got = t.state()
+    t.close()
+    assert launches < 6 * 60
+    monkeypatch.setenv("TRG_SHELL_OVERLAP", "0")
+    _, ref = steps(tp, ic, form, 6)
+    scale = np.abs(ref.U).max(axis=1, keepdims=True) + 1e-300
+    assert np.all(np.abs(got.U - ref.U) <= (0 if form == torch_b200.PRECISION_FP64 else 1e-11) * scale)

@@ -349,8 +349,12 @@ __device__ __forceinline__ void neighbours(const Params& P, const SweepCell& c, 
 	}
 	const double x0 = pick3(c.x[0], c.x[1], c.x[2], r0), x1 = pick3(c.x[0], c.x[1], c.x[2], r1);
 #ifdef TRG_FAST_MATH
+	// one division; a neighbour level with the cell where the axes tie has a
+	// weight of exactly 0 (it belongs to the cell's own shell), which the
+	// rounded reciprocal would not give
 	const double inv2 = (double)s2 / (double)e2;
-	const double ic0 = x0 - 0.5 * ((double)e0 * inv2), ic1 = x1 - 0.5 * ((double)e1 * inv2);
+	const double ic0 = x0 - 0.5 * (abs(e0) == abs(e2) ? (double)s0 : (double)e0 * inv2);
+	const double ic1 = x1 - 0.5 * (abs(e1) == abs(e2) ? (double)s1 : (double)e1 * inv2);
 #else
 	const double ic0 = x0 - 0.5 * ((double)(s2 * e0) / (double)e2);
 	const double ic1 = x1 - 0.5 * ((double)(s2 * e1) / (double)e2);
