@@ -52,19 +52,22 @@ __device__ __forceinline__ void face_ids(const Params& P, const int* ijk, int di
 __device__ __forceinline__ void hydro_udot(const Params& P, const State& S, long long id, const int* ijk, const double* xc,
                                            const double* Ubase, double* udot) {
 	double vol = cell_volume(P, xc[0]);
+	Recip rv;
+	rv.set(vol);
 #pragma unroll
 	for (int i = 0; i < NU; ++i) udot[i] = 0;
 	#pragma unroll
 	for (int dim = 0; dim < 3; ++dim) if (dim < P.nd) {
 		long long fl, fr;
 		face_ids(P, ijk, dim, fl, fr);
-		double al = face_area(P, xc, dim, 0), ar = face_area(P, xc, dim, 1);
+		const double al = rv.div(face_area(P, xc, dim, 0));
+		const double ar = P.geometry == G_CART ? al : rv.div(face_area(P, xc, dim, 1));
 		const double* Fd = S.F[dim];
 		long long nf = S.nfaces[dim];
 #pragma unroll
 		for (int i = 0; i < NU; ++i) {
-			udot[i] += (al / vol) * Fd[(long long)i * nf + fl];
-			udot[i] -= (ar / vol) * Fd[(long long)i * nf + fr];
+			udot[i] += al * Fd[(long long)i * nf + fl];
+			udot[i] -= ar * Fd[(long long)i * nf + fr];
 		}
 	}
 	for (int i = 0; i < 3; ++i) {
@@ -1790,18 +1793,23 @@ __global__ void __launch_bounds__(256) k_heating_arrays_fp64(Params P, State S) 
 // ----------------------------------------------------------------- time step
 __device__ __forceinline__ unsigned long long dbits(double v) { return (unsigned long long)__double_as_longlong(v); }
 
-__device__ __forceinline__ double block_min(double v) {
-	__shared__ double red[32];
-	for (int o = 16; o > 0; o >>= 1) v = smin(v, __shfl_down_sync(0xffffffffu, v, o));
-	int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-	if (lane == 0) red[wid] = v;
+// The block's minima of three values at once (the three chains of shuffles
+// overlap), in thread 0.
+__device__ __forceinline__ void block_min3(double* v) {
+	__shared__ double red[3][8];
+	const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
+	for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+		for (int k = 0; k < 3; ++k) v[k] = smin(v[k], __shfl_down_sync(0xffffffffu, v[k], o));
+	if (lane == 0)
+#pragma unroll
+		for (int k = 0; k < 3; ++k) red[k][wid] = v[k];
 	__syncthreads();
-	if (wid == 0) {
-		int nw = (blockDim.x + 31) >> 5;
-		v = lane < nw ? red[lane] : 1.0e308;
-		for (int o = 16; o > 0; o >>= 1) v = smin(v, __shfl_down_sync(0xffffffffu, v, o));
-	}
-	return v;
+	if (threadIdx.x == 0)
+		for (int w = 1; w < (int)blockDim.x / 32; ++w)
+#pragma unroll
+			for (int k = 0; k < 3; ++k) v[k] = smin(v[k], red[k][w]);
 }
 
 // Hydrodynamics::calculateTimeStep (Hydro.cpp:77-89), Radiation::calculateTimeStep
@@ -1852,16 +1860,19 @@ struct DtMin {
 	double inv_t, rad, thermo;
 };
 __device__ __forceinline__ void dt_cell(const Params& P, const State& S, long long id, long long first_cell,
-                                        const double* inv_dx, DtMin& m) {
+                                        const Recip& inv_dx, DtMin& m) {
 	double q_den = FLD(S.Q, DEN, id), q_pre = FLD(S.Q, PRE, id), q_hii = FLD(S.Q, HII, id);
 	double inv_t = 0;
 	double ss = sqrt(P.gamma * q_pre / q_den);
 	#pragma unroll
+	for (int dim = 0; dim < 3; ++dim) if (dim < P.nd) {
+		const double speed = fabs(FLD(S.Q, VEL + dim, id)) + ss;
 #ifdef TRG_FAST_MATH
-	for (int dim = 0; dim < 3; ++dim) if (dim < P.nd) inv_t += (fabs(FLD(S.Q, VEL + dim, id)) + ss) * inv_dx[dim];
+		inv_t += speed * inv_dx.y;
 #else
-	for (int dim = 0; dim < 3; ++dim) if (dim < P.nd) inv_t += (fabs(FLD(S.Q, VEL + dim, id)) + ss) / P.dx[dim];
+		inv_t += inv_dx.div(speed);
 #endif
+	}
 	if (inv_t == 0) inv_t = 1.0 / P.dt_max;
 	m.inv_t = smax(m.inv_t, inv_t);
 	int ijk[3];
@@ -1919,22 +1930,17 @@ __device__ __forceinline__ void b_dt_reduce_fp64(const Params& P, const State& S
 		cm = dd_prod(FLD(S.U, DEN, id), vol);
 		ce = dd_prod(FLD(S.U, PRE, id), vol);
 	}
-	double inv_dx[3];
-#pragma unroll
-	for (int dim = 0; dim < 3; ++dim) inv_dx[dim] = dim < P.nd ? 1.0 / P.dx[dim] : 0.0;
+	Recip inv_dx;
+	inv_dx.set(P.dx[0]);  // the same in every dimension (Grid.cpp:470-471)
 #pragma unroll 1
 	for (; id < P.N; id += stride) dt_cell(P, S, id, first_cell, inv_dx, m);
 	if (cons_part) block_cons_partial(cm, ce, cons_part, blockIdx.x);
-	double th = block_min(m.inv_t > 0 ? 0.5 / m.inv_t : 1.0e308);
-	__syncthreads();
-	double tr = block_min(m.rad);
-	__syncthreads();
-	double tt = block_min(m.thermo);
+	double v[3] = {m.inv_t > 0 ? 0.5 / m.inv_t : 1.0e308, m.rad, m.thermo};
+	block_min3(v);
 	if (threadIdx.x == 0) {
 		unsigned long long* slots = reinterpret_cast<unsigned long long*>(S.scal + 2);
-		atomicMin(&slots[0], dbits(th));
-		atomicMin(&slots[1], dbits(tr));
-		atomicMin(&slots[2], dbits(tt));
+#pragma unroll
+		for (int k = 0; k < 3; ++k) atomicMin(&slots[k], dbits(v[k]));
 	}
 }
 

@@ -1,39 +1,8 @@
-// A cell's part of the radiation sweep with its divisions and exponentials
-// overlapped: what the sweeps walked by one CTA (sweep_chain.cuh) and the plain
+// A cell's part of the radiation sweep with its divisions (Recip,
+// trg_device.cuh) and exponentials overlapped: what the sweeps walked by one CTA (sweep_chain.cuh) and the plain
 // per-shell kernel run.  Included by kernels_fp64.cu inside its build's
 // namespace.  Results are those of rad_shell's general loop: bit for bit in the
 // exact build.
-
-// Division by one divisor: a reciprocal by Newton's iteration, then a / b by
-// two corrections with exact remainders (P. Markstein, "Computation of
-// elementary functions on the IBM RISC System/6000 processor", IBM J. R&D 34,
-// 1990): with y the correctly rounded reciprocal, which its last iteration
-// gives unless b's significand is all ones, and a quotient within one ulp,
-// fma(remainder, y, quotient) is a / b rounded to nearest.  Operands outside
-// 2^-500 .. 2^500 (where a remainder or a quotient could leave the normal
-// range) and such divisors take the built-in division.
-struct Recip {
-	double b, y;
-	bool ok;
-	__device__ __forceinline__ static bool mid(double v) {  // 2^-500 <= |v| < 2^500
-		return (unsigned)(__double2hiint(v) & 0x7fffffff) - 0x20b00000u < 0x3e800000u;
-	}
-	__device__ __forceinline__ void set(double divisor) {
-		b = divisor;
-		ok = mid(b) && __double2loint(b) != -1;
-		asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-		y = fma(y, fma(-b, y, 1.0), y);
-		y = fma(y, fma(-b, y, 1.0), y);
-		y = fma(y, fma(-b, y, 1.0), y);
-	}
-	__device__ __forceinline__ double quotient(double a) const {
-		double q = a * y;
-		q = fma(fma(-b, q, a), y, q);
-		return fma(fma(-b, q, a), y, q);
-	}
-	__device__ __forceinline__ bool takes(double a) const { return ok && (mid(a) || a == 0.0); }
-	__device__ __forceinline__ double div(double a) const { return takes(a) ? quotient(a) : a / b; }
-};
 
 // tau_interp of two sets of optical depths at once.
 __device__ __forceinline__ void tau_interp2(const Params& P, const double* ta, const double* tb, const double* w0,

@@ -274,6 +274,7 @@ std::string host_setup(const trg_params& p, const double* den, const double* pre
 	P.photonEnergy = photonEnergy;
 	P.photonRate = photonRate;
 	P.gamma = p.gamma;
+	P.gm1_rcp = 1.0 / (p.gamma - 1.0);
 	P.X = p.mass_frac_h;
 	P.nd = p.nd;
 	P.nx = slab ? slab->nx : p.ncells[0]; P.ny = p.ncells[1]; P.nz = p.ncells[2];

@@ -15,7 +15,7 @@
 //    barrier, the neighbours' values and what follows from them are in the
 //    chain;
 //  * divisions are formed without the branch of the built-in one, so that
-//    independent ones overlap (Recip, rad_solve.cuh), and those by a divisor known before
+//    independent ones overlap (Recip, trg_device.cuh), and those by a divisor known before
 //    the neighbours are cost five operations.
 // Measured (B200, radiation / column-density sweep, per-shell launches ->
 // this): 150 x 200 grid, exact build 1203 -> 451 / 668 -> 127 us, fast build

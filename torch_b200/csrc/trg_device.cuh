@@ -40,6 +40,40 @@ namespace trg {
 __device__ __forceinline__ double smin(double a, double b) { return (b < a) ? b : a; }
 __device__ __forceinline__ double smax(double a, double b) { return (a < b) ? b : a; }
 
+// Division by one divisor: a reciprocal by Newton's iteration, then a / b by
+// two corrections with exact remainders (P. Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", IBM J. R&D 34,
+// 1990): with y the correctly rounded reciprocal, which its last iteration
+// gives unless b's significand is all ones, and a quotient within one ulp,
+// fma(remainder, y, quotient) is a / b rounded to nearest.  Operands outside
+// 2^-500 .. 2^500 (where a remainder or a quotient could leave the normal
+// range) and such divisors take the built-in division.  It has no branch where
+// several quotients are tested together (takes), so that they overlap, and
+// costs five operations per quotient once the reciprocal is there; the built-in
+// one is a serial 112 cycles each, and more where the numerator is 0.
+struct Recip {
+	double b, y;
+	bool ok;
+	__device__ __forceinline__ static bool mid(double v) {  // 2^-500 <= |v| < 2^500
+		return (unsigned)(__double2hiint(v) & 0x7fffffff) - 0x20b00000u < 0x3e800000u;
+	}
+	__device__ __forceinline__ void set(double divisor) {
+		b = divisor;
+		ok = mid(b) && __double2loint(b) != -1;
+		asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+		y = fma(y, fma(-b, y, 1.0), y);
+		y = fma(y, fma(-b, y, 1.0), y);
+		y = fma(y, fma(-b, y, 1.0), y);
+	}
+	__device__ __forceinline__ double quotient(double a) const {
+		double q = a * y;
+		q = fma(fma(-b, q, a), y, q);
+		return fma(fma(-b, q, a), y, q);
+	}
+	__device__ __forceinline__ bool takes(double a) const { return ok && (mid(a) || a == 0.0); }
+	__device__ __forceinline__ double div(double a) const { return takes(a) ? quotient(a) : a / b; }
+};
+
 __device__ __forceinline__ void cell_ijk(const Params& P, long long id, int* ijk) {
 	if (P.N <= 0x7fffffffLL) {  // two multiplications instead of the 64-bit divisions
 		const unsigned u = (unsigned)id;
@@ -148,16 +182,35 @@ __device__ __forceinline__ void UfromQ(double* u, const double* q, double gamma,
 }
 
 __device__ __forceinline__ void QfromU(double* q, const double* u, double gamma, int nd) {
-	q[DEN] = u[DEN];
-	double ke = 0;
+	Recip r;
+	r.set(u[DEN]);
+	double k[3] = {0, 0, 0};
+	bool ok = r.takes(u[HII]) && r.takes(u[ADV]);
 	#pragma unroll
 	for (int dim = 0; dim < 3; ++dim) if (dim < nd) {
-		q[VEL + dim] = u[VEL + dim] / u[DEN];
-		ke += 0.5 * u[VEL + dim] * u[VEL + dim] / u[DEN];
+		k[dim] = 0.5 * u[VEL + dim] * u[VEL + dim];
+		ok &= r.takes(u[VEL + dim]) && r.takes(k[dim]);
+	}
+	q[DEN] = u[DEN];
+	double ke = 0;
+	if (ok) {
+		#pragma unroll
+		for (int dim = 0; dim < 3; ++dim) if (dim < nd) {
+			q[VEL + dim] = r.quotient(u[VEL + dim]);
+			ke += r.quotient(k[dim]);
+		}
+		q[HII] = r.quotient(u[HII]);
+		q[ADV] = r.quotient(u[ADV]);
+	} else {
+		#pragma unroll
+		for (int dim = 0; dim < 3; ++dim) if (dim < nd) {
+			q[VEL + dim] = u[VEL + dim] / u[DEN];
+			ke += k[dim] / u[DEN];
+		}
+		q[HII] = u[HII] / u[DEN];
+		q[ADV] = u[ADV] / u[DEN];
 	}
 	q[PRE] = (u[PRE] - ke) * (gamma - 1.0);
-	q[HII] = u[HII] / u[DEN];
-	q[ADV] = u[ADV] / u[DEN];
 }
 
 __device__ __forceinline__ void FfromQ(double* f, const double* q, double gamma, int nd, int dim) {
@@ -187,6 +240,18 @@ __device__ __forceinline__ double calc_temperature(const Params& P, double hii, 
 #endif
 }
 
+// temperature = pre / x < T_floor as rounded, divided only next to the floor.
+__device__ __forceinline__ bool below_tfloor(const Params& P, double pre, double x) {
+	if (pre > 1.0000001 * (P.tfloor * x)) return false;
+	return pre / x < P.tfloor;
+}
+// a / (gamma - 1) with the host's correctly rounded reciprocal.
+__device__ __forceinline__ double over_gm1(const Params& P, double a) {
+	const double b = P.gamma - 1.0;
+	const Recip r = {b, P.gm1_rcp, Recip::mid(b)};
+	return r.div(a);
+}
+
 // Fluid::fixPrimitives for one cell, Fluid.cpp:138-150 (floor uses U[DEN]).
 __device__ __forceinline__ void fix_primitives(const Params& P, double* q, double u_den) {
 	q[HII] = smax(smin(q[HII], 1.0), 0.0);
@@ -194,8 +259,7 @@ __device__ __forceinline__ void fix_primitives(const Params& P, double* q, doubl
 	q[DEN] = smax(q[DEN], P.dfloor);
 	q[PRE] = smax(q[PRE], P.pfloor);
 	double mu_inv = P.X * (q[HII] + 1.0) + (1.0 - P.X) * 0.25;
-	double temperature = q[PRE] / (mu_inv * P.specificGasConstant * q[DEN]);
-	if (temperature < P.tfloor)
+	if (below_tfloor(P, q[PRE], mu_inv * P.specificGasConstant * q[DEN]))
 		q[PRE] = mu_inv * P.specificGasConstant * u_den * P.tfloor;
 }
 
@@ -203,24 +267,37 @@ __device__ __forceinline__ void fix_primitives(const Params& P, double* q, doubl
 // conditions under which the reference throws.
 __device__ __forceinline__ bool fix_solution(const Params& P, double* u) {
 	if (!isfinite(u[DEN]) || !isfinite(u[PRE])) return false;
-	double hii = smax(smin(u[HII] / u[DEN], 1.0), 0.0);
-	double adv = smax(smin(u[ADV] / u[DEN], 1.0), 0.0);
-	double v[3] = {0, 0, 0};
-	double den = smax(u[DEN], P.dfloor);
+	Recip r;
+	r.set(u[DEN]);
+	bool ok = r.takes(u[HII]) && r.takes(u[ADV]);
 	#pragma unroll
-	for (int dim = 0; dim < 3; ++dim) if (dim < P.nd) v[dim] = u[VEL + dim] / u[DEN];
+	for (int dim = 0; dim < 3; ++dim) if (dim < P.nd) ok &= r.takes(u[VEL + dim]);
+	double hii, adv, v[3] = {0, 0, 0};
+	if (ok) {
+		hii = r.quotient(u[HII]);
+		adv = r.quotient(u[ADV]);
+		#pragma unroll
+		for (int dim = 0; dim < 3; ++dim) if (dim < P.nd) v[dim] = r.quotient(u[VEL + dim]);
+	} else {
+		hii = u[HII] / u[DEN];
+		adv = u[ADV] / u[DEN];
+		#pragma unroll
+		for (int dim = 0; dim < 3; ++dim) if (dim < P.nd) v[dim] = u[VEL + dim] / u[DEN];
+	}
+	hii = smax(smin(hii, 1.0), 0.0);
+	adv = smax(smin(adv, 1.0), 0.0);
+	double den = smax(u[DEN], P.dfloor);
 	double ke = 0.0;
 	#pragma unroll
 	for (int dim = 0; dim < 3; ++dim) if (dim < P.nd) ke += v[dim] * v[dim];
 	ke *= 0.5 * u[DEN];
 	double pre = (u[PRE] - ke) * (P.gamma - 1.0);
-	ke *= den / u[DEN];
+	if (den != u[DEN]) ke *= den / u[DEN];
 	if (pre < P.pfloor) pre = P.pfloor;
 	double mu_inv = P.X * (hii + 1.0) + (1.0 - P.X) * 0.25;
-	double temperature = pre / (mu_inv * P.specificGasConstant * den);
-	if (temperature < P.tfloor) pre = mu_inv * P.specificGasConstant * den * P.tfloor;
+	if (below_tfloor(P, pre, mu_inv * P.specificGasConstant * den)) pre = mu_inv * P.specificGasConstant * den * P.tfloor;
 	u[DEN] = den;
-	u[PRE] = pre / (P.gamma - 1.0) + ke;
+	u[PRE] = over_gm1(P, pre) + ke;
 	u[HII] = hii * den;
 	u[ADV] = adv * den;
 	#pragma unroll

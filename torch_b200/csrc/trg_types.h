@@ -121,6 +121,7 @@ struct Params {
 	int riemann, limiter;
 	double dx[3];
 	double gamma, X;
+	double gm1_rcp;  // 1 / (gamma - 1)
 	double hydrogenMass, specificGasConstant, boltzmannConst, rydbergEnergy, dustXsec, pi;
 	double voronov_A, voronov_X, voronov_K, voronov_P, voronov_DE;
 	double dt_max, dfloor, pfloor, tfloor;
