@@ -73,3 +73,18 @@ def test_time_step_with_many_cells_per_thread(form):
     dts, got = run(tp, ic, form, 4)
     ref_dts, ref = run(tp, ic, form, 4, lambda t: t.conservation_enable(True))
     assert np.array_equal(dts, ref_dts) and np.array_equal(got.U, ref.U)
+
+
+@pytest.mark.parametrize("form", FORMS)
+@pytest.mark.parametrize("case", ["hydro_2d", "hydro_3d", "hii"])
+def test_overlapped_launches_equal_serial_ones(monkeypatch, form, case):
+    """Kernels launched while the one before them still runs wait for it before
+    they read anything (TRG_SHELL_OVERLAP=0 launches them one after another)."""
+    if case == "hii":
+        tp, ic = workloads.hii_region(n=24, seed=8)
+    else:
+        tp, ic = workloads.sedov(n=40, nd=2 if case == "hydro_2d" else 3)
+    dts, got = run(tp, ic, form, 30)
+    monkeypatch.setenv("TRG_SHELL_OVERLAP", "0")
+    ref_dts, ref = run(tp, ic, form, 30)
+    assert np.array_equal(dts, ref_dts) and np.array_equal(got.U, ref.U) and np.array_equal(got.Q, ref.Q)

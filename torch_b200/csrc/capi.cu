@@ -102,6 +102,8 @@ struct trg_ctx {
 	// (programmatic dependent launch), and small grids walk all of them in one
 	// launch; TRG_SHELL_OVERLAP=0 launches them one after another
 	bool shell_overlap = shell_overlap_default();
+	// a batch's whole step is being captured (with its side stream's joins)
+	bool step_capture = false;
 	// sweeps as one launch (sweep_chain.cuh): threads per CTA (0: a launch per
 	// shell) and dynamic shared memory
 	struct ChainShape {
@@ -204,13 +206,31 @@ void profile_collect(trg_ctx* c) {
 // the exact or the fast build of a kernels_fp64.cu kernel, by the context's form
 #define KF(name) (c->fastk == 1 ? trg::fast::name : (c->fastk == 2 ? trg::fastb::name : trg::exact::name))
 
+// A kernel of the step.  It may be launched before the one ahead of it in the
+// stream has finished (programmatic stream serialisation; every kernel given
+// to it starts with grid_begin, which waits), so that its launch, about 1 us,
+// is not part of the chain of small kernels that a step of a small grid is.
+template <typename... KArgs, typename... Args>
+void launch_next(trg_ctx* c, void (*kernel)(KArgs...), long long n, int block, size_t smem, Args... args) {
+	cudaLaunchConfig_t cfg = {};
+	cfg.gridDim = dim3(grid_for(n, block));
+	cfg.blockDim = dim3(block);
+	cfg.dynamicSmemBytes = smem;
+	cfg.stream = c->stream;
+	cudaLaunchAttribute attr[1];
+	attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+	attr[0].val.programmaticStreamSerializationAllowed = 1;
+	cfg.attrs = attr;
+	cfg.numAttrs = c->shell_overlap && !c->step_capture ? 1 : 0;
+	cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
 #define LAUNCH(kernel, n, block, ...)                                                        \
 	do {                                                                                     \
 		if ((n) > 0) {                                                                       \
 			cudaEvent_t ea_ = nullptr, eb_ = nullptr;                                        \
 			if (c->profiling) { ea_ = pool_event(c); eb_ = pool_event(c);                    \
 			                    cudaEventRecord(ea_, c->stream); }                           \
-			kernel<<<grid_for((n), (block)), (block), 0, c->stream>>>(__VA_ARGS__);          \
+			launch_next(c, kernel, (n), (block), 0, __VA_ARGS__);                            \
 			if (c->profiling) { cudaEventRecord(eb_, c->stream);                             \
 			                    c->recs.push_back({#kernel, ea_, eb_}); }                    \
 			c->launches++;                                                                   \
@@ -329,7 +349,7 @@ void launch_chain(trg_ctx* c, const char* name, void (*kernel)(KArgs...), const 
 	cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem);
 	cudaEvent_t ea = nullptr, eb = nullptr;
 	if (c->profiling) { ea = pool_event(c); eb = pool_event(c); cudaEventRecord(ea, c->stream); }
-	kernel<<<c->nscalar, sh.threads, sh.smem, c->stream>>>(args...);
+	launch_next(c, kernel, (long long)c->nscalar * sh.threads, sh.threads, sh.smem, args...);
 	if (c->profiling) { cudaEventRecord(eb, c->stream); c->recs.push_back({name, ea, eb}); }
 	c->launches++;
 }
@@ -862,8 +882,8 @@ int build_chain(trg_ctx* c, const std::vector<long long>& off, const int* d_cell
 	CUDA_TRY(cudaMemsetAsync(bad, 0, sizeof(int), c->stream));
 	int* pos = reinterpret_cast<int*>(c->S.UDOT);  // zero between uses
 	CUDA_TRY(cudaMemsetAsync(pos, 0xff, c->P.N * sizeof(int), c->stream));
-	LAUNCH(KF(k_chain_positions), ch.n, 256, d_cells, ch.n, pos);
-	LAUNCH(KF(k_chain_tables), ch.n, 256, c->P, ch, pos, rad ? 1 : 0, slot, w, bad);
+	KF(k_chain_positions)<<<grid_for(ch.n, 256), 256, 0, c->stream>>>(d_cells, ch.n, pos);
+	KF(k_chain_tables)<<<grid_for(ch.n, 256), 256, 0, c->stream>>>(c->P, ch, pos, rad ? 1 : 0, slot, w, bad);
 	CUDA_TRY(cudaMemsetAsync(pos, 0, c->P.N * sizeof(int), c->stream));
 	int h_bad = 0;
 	CUDA_TRY(cudaMemcpyAsync(&h_bad, bad, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
@@ -1049,7 +1069,7 @@ int create_impl(const trg_params* p, const SlabSpec* slab, const double* den, co
 		c->fastk = 1;
 		c->zchunk = ctx_fp32_zchunk(c);
 		if ((rc = dalloc(c, &c->U32, 7 * N)) || (rc = dalloc(c, &c->U32s, 7 * N))) return rc;
-		LAUNCH(k_f64_to_f32, 7 * N, 256, c->P, S.U, c->U32);
+		k_f64_to_f32<<<grid_for(7 * N, 256), 256, 0, st>>>(c->P, S.U, c->U32);
 		CUDA_TRY(cudaMemsetAsync(c->U32s, 0, 7 * N * sizeof(float), st));
 	}
 	// TRG_FP64_KERNELS=exact|fast, read when a context is created: the build of
@@ -1292,7 +1312,7 @@ int trg_get_state(trg_ctx* c, double* U, double* Q, double* R, double* T, double
 	cudaStream_t st = c->stream;
 	if (c->fp32) {
 		// expose the FP32 state as FP64 (Q = QfromU without floors)
-		LAUNCH(k_f32_to_f64, 7 * N, 256, c->P, c->U32, c->S.U);
+		k_f32_to_f64<<<grid_for(7 * N, 256), 256, 0, st>>>(c->P, c->U32, c->S.U);
 		q_from_u(c, 0, 0);
 	}
 	if (U) CUDA_TRY(cudaMemcpyAsync(U, c->S.U, 7 * N * sizeof(double), cudaMemcpyDeviceToHost, st));
@@ -1310,7 +1330,7 @@ int trg_set_conserved(trg_ctx* c, const double* U) {
 	c->q_fresh = false;
 	c->colden_valid = false;
 	CUDA_TRY(cudaMemcpyAsync(c->S.U, U, 7 * c->P.N * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-	if (c->fp32) LAUNCH(k_f64_to_f32, 7 * c->P.N, 256, c->P, c->S.U, c->U32);
+	if (c->fp32) k_f64_to_f32<<<grid_for(7 * c->P.N, 256), 256, 0, c->stream>>>(c->P, c->S.U, c->U32);
 	return TRG_OK;
 }
 
@@ -1995,7 +2015,9 @@ void batch_step(trg_batch* b, double dt_next) {
 	cudaGraph_t graph = nullptr;
 	bool captured = false;
 	if (cudaStreamBeginCapture(v->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
+		v->step_capture = true;
 		enqueue_full_step(v, dt_next);
+		v->step_capture = false;
 		captured = cudaStreamEndCapture(v->stream, &graph) == cudaSuccess && graph;
 	}
 	v->use_graphs = use_graphs;

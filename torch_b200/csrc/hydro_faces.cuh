@@ -524,6 +524,7 @@ __device__ __forceinline__ void one_face_of(const Params& P, const State& S, lon
 }
 // Every face of a batch along dim.
 __global__ void __launch_bounds__(128) k_faces_batch_fp64(Params P, State S, int dim) {
+	grid_begin();
 #if TRG_BATCHED
 	const BatchTable& B = *P.batch;
 	const long long* off = B.face_off[dim];
@@ -552,6 +553,15 @@ __device__ __forceinline__ void all_faces(const Params& P, const State& S, const
 		if (ND > 2 && c * G.chunk <= P.nz) faces_column<2, ND>(P, S, t - c * cols, (int)c * G.chunk, G.chunk);
 	}
 }
-__global__ void __launch_bounds__(128) k_faces1_fp64(Params P, State S, FaceGrid G) { all_faces<1>(P, S, G); }
-__global__ void __launch_bounds__(128, 4) k_faces2_fp64(Params P, State S, FaceGrid G) { all_faces<2>(P, S, G); }
-__global__ void __launch_bounds__(128, 4) k_faces3_fp64(Params P, State S, FaceGrid G) { all_faces<3>(P, S, G); }
+__global__ void __launch_bounds__(128) k_faces1_fp64(Params P, State S, FaceGrid G) {
+	grid_begin();
+	all_faces<1>(P, S, G);
+}
+__global__ void __launch_bounds__(128, 4) k_faces2_fp64(Params P, State S, FaceGrid G) {
+	grid_begin();
+	all_faces<2>(P, S, G);
+}
+__global__ void __launch_bounds__(128, 4) k_faces3_fp64(Params P, State S, FaceGrid G) {
+	grid_begin();
+	all_faces<3>(P, S, G);
+}

@@ -1080,6 +1080,7 @@ template <int STAGE, typename TS, int LIM, int RS>
 __global__ void __launch_bounds__(BX* BY, 2)
     k_hydro_stage_fp32(Params P, State S, const TS* __restrict__ Uq, const TS* Ubase, TS* Uout, double hfac,
                        int zchunk, const __grid_constant__ CUtensorMap tmap, int use_tma) {
+	grid_begin();
 	hydro_stage_body<STAGE, TS, LIM, RS>(P, S, Uq, Ubase, Uout, hfac, zchunk, &tmap, use_tma, blockIdx.x, blockIdx.y,
 	                                     blockIdx.z);
 }
@@ -1173,8 +1174,17 @@ static void launch_one(const Params& P, const State& S, const TS* Uq, const TS* 
 		use_tma = state_tensor_map(P, reinterpret_cast<const double*>(Uq), &tmap) ? 1 : 0;
 	cudaFuncSetAttribute(k_hydro_stage_fp32<STAGE, TS, LIM, RS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
 	                     (int)smem);
-	k_hydro_stage_fp32<STAGE, TS, LIM, RS><<<grid, BX * BY, smem, stream>>>(P, S, Uq, Ubase, Uout, hfac, zc, tmap,
-	                                                                         use_tma);
+	cudaLaunchConfig_t cfg = {};
+	cfg.gridDim = grid;
+	cfg.blockDim = dim3(BX * BY);
+	cfg.dynamicSmemBytes = smem;
+	cfg.stream = stream;
+	cudaLaunchAttribute attr[1];  // grid_begin
+	attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+	attr[0].val.programmaticStreamSerializationAllowed = 1;
+	cfg.attrs = attr;
+	cfg.numAttrs = 1;
+	cudaLaunchKernelEx(&cfg, k_hydro_stage_fp32<STAGE, TS, LIM, RS>, P, S, Uq, Ubase, Uout, hfac, zc, tmap, use_tma);
 }
 
 // the reference's configured and default pair (albada, RotatedHLLC) is compiled

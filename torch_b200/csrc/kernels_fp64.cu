@@ -149,6 +149,7 @@ __device__ __forceinline__ void b_hydro_update_fp64(const Params& P, const State
 }
 __global__ void __launch_bounds__(256) k_hydro_update_fp64(Params P, State S, double h, int sel_base, int sel_out,
                                                           int mode) {
+	grid_begin();
 	if (TRG_BATCHED && P.batch) {
 		const BatchTable& B = *P.batch;
 		const int g = batch_slot(B.cell_off, B.G, blockIdx.x * (long long)blockDim.x);
@@ -183,6 +184,7 @@ __device__ __forceinline__ void b_q_from_u_fp64(const Params& P, const State& S,
 	if (bad) atomicOr(S.err, ERRB_NAN);
 }
 __global__ void __launch_bounds__(256) k_q_from_u_fp64(Params P, State S, int sel_src, int fix) {
+	grid_begin();
 	if (TRG_BATCHED && P.batch) {
 		const BatchTable& B = *P.batch;
 		const int g = batch_slot(B.cell_off, B.G, blockIdx.x * (long long)blockDim.x);
@@ -207,6 +209,7 @@ __device__ __forceinline__ void b_advance_fp64(const Params& P, const State& S, 
 	for (int i = 0; i < NU; ++i) FLD(S.U, i, id) = u[i];
 }
 __global__ void __launch_bounds__(256) k_advance_fp64(Params P, State S, double dt) {
+	grid_begin();
 	if (TRG_BATCHED && P.batch) {
 		const BatchTable& B = *P.batch;
 		const int g = batch_slot(B.cell_off, B.G, blockIdx.x * (long long)blockDim.x);
@@ -480,6 +483,7 @@ __device__ __forceinline__ void b_rad_wind_reset(const Params& P, const State& S
 	RFLD(S.R, R_HII_A, id) = 1;
 }
 __global__ void k_rad_wind_reset(Params P, State S, const int* __restrict__ cells, int count) {
+	grid_begin();
 	const int t = blockIdx.x * blockDim.x + threadIdx.x;
 	if (t >= count) return;
 	if (TRG_BATCHED && P.batch) {
@@ -863,6 +867,7 @@ __device__ __forceinline__ void b_rad_sweep_prep(const Params& P, const State& S
                                                  int init);
 __global__ void __launch_bounds__(256) k_rad_sweep_prep(Params P, State S, const int* __restrict__ cells, int n,
                                                          int init) {
+	grid_begin();
 	if (TRG_BATCHED && P.batch) {  // grids whose sweep is a chain (no learned start)
 		const BatchTable& B = *P.batch;
 		const int g = batch_slot(B.cell_off, B.G, blockIdx.x * (long long)blockDim.x);
@@ -1001,6 +1006,7 @@ __global__ void TRG_RAD_SHELL_BOUNDS k_rad_shell_fp64_ls(Params P, State S, cons
 // every candidate's slot.  One thread per cell of the padded ranges (a
 // 256-thread block never straddles two grids).
 __global__ void __launch_bounds__(256) k_batch_learned_prep(Params Pv, State Sv) {
+	grid_begin();
 #if TRG_BATCHED
 	const BatchTable& B = *Pv.batch;
 	const long long pos = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -1111,6 +1117,7 @@ __device__ __forceinline__ void b_rad_solve2(const Params& P, const State& S, lo
 }
 __global__ void __launch_bounds__(128) k_rad_solve2(Params P, State S, const int* __restrict__ cells, int count,
                                                     double h) {
+	grid_begin();
 	const int t = blockIdx.x * blockDim.x + threadIdx.x;
 	if (t >= count) return;
 	if (TRG_BATCHED && P.batch) {
@@ -1134,6 +1141,7 @@ __device__ __forceinline__ void b_rad_no_star_fp64(const Params& P, const State&
 	FLD(S.Q, HII, id) = x_new;
 }
 __global__ void k_rad_no_star_fp64(Params P, State S, double h) {
+	grid_begin();
 	if (TRG_BATCHED && P.batch) {
 		const BatchTable& B = *P.batch;
 		const int g = batch_slot(B.cell_off, B.G, blockIdx.x * (long long)blockDim.x);
@@ -1163,6 +1171,7 @@ __device__ __forceinline__ void b_rad_heating_fp64(const Params& P, const State&
 	rad_heating_cell(P, S, id, q_hii, FLD(S.Q, PRE, id), FLD(S.Q, DEN, id));
 }
 __global__ void __launch_bounds__(256) k_rad_heating_fp64(Params P, State S) {
+	grid_begin();
 	if (TRG_BATCHED && P.batch) {
 		const BatchTable& B = *P.batch;
 		const int g = batch_slot(B.cell_off, B.G, blockIdx.x * (long long)blockDim.x);
@@ -1211,6 +1220,7 @@ __device__ __forceinline__ void b_rad_update_fp64(const Params& P, const State& 
 	if (mode == 2) store_q<true>(P, S, id, u);
 }
 __global__ void __launch_bounds__(256) k_rad_update_fp64(Params P, State S, double h, int mode) {
+	grid_begin();
 	if (TRG_BATCHED && P.batch) {
 		const BatchTable& B = *P.batch;
 		const int g = batch_slot(B.cell_off, B.G, blockIdx.x * (long long)blockDim.x);
@@ -1267,6 +1277,7 @@ __device__ __forceinline__ void b_rad_update_lean(const Params& P, const State& 
 	FLD(S.Q, ADV, id) = adv;
 }
 __global__ void __launch_bounds__(256) k_rad_update_lean(Params P, State S, double h) {
+	grid_begin();
 	if (TRG_BATCHED && P.batch) {
 		const BatchTable& B = *P.batch;
 		const int g = batch_slot(B.cell_off, B.G, blockIdx.x * (long long)blockDim.x);
@@ -1421,6 +1432,7 @@ __device__ __forceinline__ void b_colden_sweep_prep(const Params& P, const State
 }
 __global__ void __launch_bounds__(256) k_colden_sweep_prep(Params P, State S, const int* __restrict__ cells, int n,
                                                             int init) {
+	grid_begin();
 	if (TRG_BATCHED && P.batch) {  // grids whose sweep is a chain
 		const BatchTable& B = *P.batch;
 		const int g = batch_slot(B.cell_off, B.G, blockIdx.x * (long long)blockDim.x);
@@ -1486,6 +1498,7 @@ __device__ __forceinline__ void b_thermo_rates_fp64(const Params& P, const State
 	TFLD(S.T, T_RATE, id) = P.heating_amp * rate;
 }
 __global__ void __launch_bounds__(256) k_thermo_rates_fp64(Params P, State S) {
+	grid_begin();
 	if (TRG_BATCHED && P.batch) {
 		const BatchTable& B = *P.batch;
 		const int g = batch_slot(B.cell_off, B.G, blockIdx.x * (long long)blockDim.x);
@@ -1605,6 +1618,7 @@ __device__ __forceinline__ void b_thermo_integrate_fp64(const Params& P, const S
 	thermo_finish(P, S, id, c);
 }
 __global__ void __launch_bounds__(256) k_thermo_integrate_fp64(Params P, State S, double h) {
+	grid_begin();
 	if (TRG_BATCHED && P.batch) {
 		const BatchTable& B = *P.batch;
 		const int g = batch_slot(B.cell_off, B.G, blockIdx.x * (long long)blockDim.x);
@@ -1693,6 +1707,7 @@ __device__ __forceinline__ void b_thermo_update_fp64(const Params& P, const Stat
 	if (mode == 2) store_q<true>(P, S, id, u);
 }
 __global__ void __launch_bounds__(256) k_thermo_update_fp64(Params P, State S, double h, int mode) {
+	grid_begin();
 	if (TRG_BATCHED && P.batch) {
 		const BatchTable& B = *P.batch;
 		const int g = batch_slot(B.cell_off, B.G, blockIdx.x * (long long)blockDim.x);
@@ -1739,6 +1754,7 @@ __device__ __forceinline__ void b_thermo_lean(const Params& P, const State& S, l
 	TFLD(S.T, T_HEAT, id) = 0;
 }
 __global__ void __launch_bounds__(256) k_thermo_lean(Params P, State S, double h, int update_only) {
+	grid_begin();
 	if (TRG_BATCHED && P.batch) {
 		const BatchTable& B = *P.batch;
 		const int g = batch_slot(B.cell_off, B.G, blockIdx.x * (long long)blockDim.x);
@@ -1754,6 +1770,7 @@ __global__ void __launch_bounds__(256) k_thermo_lean(Params P, State S, double h
 // rayTrace (the column-density sweep, launched before), non-wind cells.
 // Single grids only.
 __global__ void __launch_bounds__(256) k_heating_arrays_fp64(Params P, State S) {
+	grid_begin();
 	const long long id = blockIdx.x * (long long)blockDim.x + threadIdx.x;
 	if (id >= P.N) return;
 	int ijk[3];
@@ -1840,6 +1857,7 @@ __device__ __forceinline__ void dt_end(const Params& P, const State& S, const Dt
 	b_dt_finalize(P, S, end.dt_next, 0, end.step);
 }
 __global__ void __launch_bounds__(256, 4) k_dt_reduce_fp64(Params P, State S, long long first_cell, DtEnd end) {
+	grid_begin();
 	if (TRG_BATCHED && P.batch) {
 		// grid ranges are padded to whole blocks: the block reduction stays within one grid
 		const BatchTable& B = *P.batch;
@@ -1973,6 +1991,7 @@ __device__ __forceinline__ void b_dt_finalize(const Params& P, const State& S, d
 	if (S.dt_hist && step >= 0) S.dt_hist[step] = dt;
 }
 __global__ void k_dt_finalize(Params P, State S, double dt_next, int first_time, int step) {
+	grid_begin();
 	if (TRG_BATCHED && P.batch) {
 		const int g = blockIdx.x * blockDim.x + threadIdx.x;
 		if (g < P.batch->G) b_dt_finalize(P.batch->P[g], P.batch->S[g], dt_next, first_time, step);
@@ -1982,7 +2001,10 @@ __global__ void k_dt_finalize(Params P, State S, double dt_next, int first_time,
 }
 // The minima from dt_max again, after a reduction whose minima the host read
 // and after a restored checkpoint (single grids).
-__global__ void k_dt_reset(Params P, State S) { b_dt_reset(P, S); }
+__global__ void k_dt_reset(Params P, State S) {
+	grid_begin();
+	b_dt_reset(P, S);
+}
 
 // ------------------------------------------- FP64 fallback of the FP32 form
 // A hydro sub-step of the FP32 form keeps FP64 arithmetic for the cells whose
@@ -2009,6 +2031,7 @@ __device__ __forceinline__ long long clamp_nb(const Params& P, const int* ijk, i
 // and y, are staged in shared memory once; the z neighbours come from a window
 // of the column's pressures kept in registers.
 __global__ void __launch_bounds__(256) k_fb_flags(Params P, State S, double contrast) {
+	grid_begin();
 	__shared__ double tile[8 + 4][32 + 4];
 	const int lane = threadIdx.x & 31, row = threadIdx.x >> 5;
 	const int x0 = blockIdx.x * 32, y0 = blockIdx.y * 8;
@@ -2086,6 +2109,7 @@ __device__ __forceinline__ void fb_faces_along(const Params& P, const State& S, 
 	}
 }
 __global__ void __launch_bounds__(128) k_fb_faces(Params P, State S) {
+	grid_begin();
 	const unsigned n = *S.fb_count;
 	if (P.nd == 3) {
 		if (blockIdx.x % 3 == 0) fb_faces_along<0, 3>(P, S, n);
@@ -2098,6 +2122,7 @@ __global__ void __launch_bounds__(128) k_fb_faces(Params P, State S) {
 }
 // FP64 update of every listed cell, U -> U1, with Q of the result.
 __global__ void __launch_bounds__(256) k_fb_update(Params P, State S, double h) {
+	grid_begin();
 	const unsigned n = *S.fb_count;
 	for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x)
 		b_hydro_update_fp64(P, S, S.fb_list[t], h, 0, 1, 2);

@@ -141,9 +141,11 @@ __device__ __forceinline__ void chain_kernel(const Params& P, const State& S, do
 	else chain_sweep<RAD>(P, S, h);
 }
 __global__ void __launch_bounds__(2 * CHAIN_GROUP, 1) k_rad_chain(Params P, State S, double h) {
+	grid_begin();
 	chain_kernel<true>(P, S, h);
 }
 __global__ void __launch_bounds__(2 * CHAIN_GROUP, 1) k_colden_chain(Params P, State S) {
+	grid_begin();
 	chain_kernel<false>(P, S, 0.0);
 }
 

@@ -32,6 +32,15 @@
 
 namespace trg {
 
+// Start of a kernel that may be launched before the one ahead of it in its
+// stream has finished (programmatic dependent launch): it waits until that one
+// has completed and its writes are visible, and lets the next one start its
+// own launch.  Returns at once in a launch without that attribute.
+__device__ __forceinline__ void grid_begin() {
+	asm volatile("griddepcontrol.wait;" ::: "memory");
+	asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 #define FLD(a, f, i) ((a)[(long long)(f) * P.N + (i)])
 // radiation and thermodynamics fields (layouts in trg_types.h)
 #define RFLD(a, f, i) ((a)[r_index(P.N, (f), (i))])
