@@ -237,9 +237,12 @@ void launch_next(trg_ctx* c, void (*kernel)(KArgs...), long long n, int block, s
 		}                                                                                    \
 	} while (0)
 
-// A shell of a causal sweep.  Every shell after the first of a sweep is
+// A shell of a causal sweep.  Every shell after the first one with cells is
 // launched with programmatic stream serialisation: its CTAs may start while
-// the previous shell runs and wait for it inside the kernel (sweep_wait).
+// the previous shell runs and wait for it inside the kernel (sweep_wait).  The
+// first one (in radiation sweeps not shell 0, which is the star's cell) starts
+// when all before it has ended: what a shell reads ahead of its wait, such as
+// the inputs in sweep order, is written by the kernels ahead of the sweep.
 template <typename... KArgs, typename... Args>
 void launch_shell(trg_ctx* c, void (*kernel)(KArgs...), int n, int block, bool overlap, Args... args) {
 	cudaLaunchConfig_t cfg = {};
@@ -372,10 +375,10 @@ void colden_sweep_direct(trg_ctx* c) {
 	for (size_t s = 0; s + 1 < off.size(); ++s) {
 		int count = (int)(off[s + 1] - off[s]);
 		if (sw)
-			LAUNCH_SHELL(KF(k_colden_shell_sw), count, 128, s > 0, c->P, c->S, c->d_sweep_all + off[s], count,
+			LAUNCH_SHELL(KF(k_colden_shell_sw), count, 128, off[s] > 0, c->P, c->S, c->d_sweep_all + off[s], count,
 			             (long long)off[s]);
 		else
-			LAUNCH_SHELL(KF(k_colden_shell_fp64), count, 128, s > 0, c->P, c->S, c->d_sweep_all + off[s], count);
+			LAUNCH_SHELL(KF(k_colden_shell_fp64), count, 128, off[s] > 0, c->P, c->S, c->d_sweep_all + off[s], count);
 	}
 }
 
@@ -512,7 +515,7 @@ void rad_sweep_direct(trg_ctx* c, double h) {
 	const auto& off = c->hs.off_nonwind;
 	for (size_t s = 0; s + 1 < off.size(); ++s) {
 		int count = (int)(off[s + 1] - off[s]);
-		rad_shell_launch(c, c->d_sweep_nonwind + off[s], count, h, s > 0, (long long)off[s]);
+		rad_shell_launch(c, c->d_sweep_nonwind + off[s], count, h, off[s] > 0, (long long)off[s]);
 	}
 }
 
@@ -524,7 +527,7 @@ void tau_sweep_direct(trg_ctx* c) {
 	const auto& off = c->hs.off_nonwind;
 	for (size_t s = 0; s + 1 < off.size(); ++s) {
 		int count = (int)(off[s + 1] - off[s]);
-		LAUNCH_SHELL(KF(k_rad_tau_shell), count, 128, s > 0, c->P, c->S, c->d_sweep_nonwind + off[s], count);
+		LAUNCH_SHELL(KF(k_rad_tau_shell), count, 128, off[s] > 0, c->P, c->S, c->d_sweep_nonwind + off[s], count);
 	}
 }
 
