@@ -931,24 +931,32 @@ namespace trg {
 const Params& ctx_params(const trg_ctx* c) { return c->P; }
 State ctx_state(const trg_ctx* c) { return c->S; }
 int ctx_device(const trg_ctx* c) { return c->raw.device; }
-// Planes per CTA of the FP32 hydro pass on this grid: a CTA's time is its
+// Planes per CTA of the FP32 hydro pass on this grid.  A CTA's time is its
 // planes and about 3.5 more (the planes before its first are loaded and one of
-// them computed), and two CTAs fit on an SM, so the grid takes
-// ceil(CTAs / 2 SMs) times that (a wave that is 6% over still ends with the
-// others).  Measured per launch against a fixed least depth of 16 (64 CTAs on
-// 148 SMs at 64^3): 32^3 137 -> 31 us, 64^3 142 -> 57, 75^3 143 -> 96 (FP64 state
-// 198 -> 138), 96^3 154 -> 128, 100^3 (FP64 state) 381 -> 282; the choice is within
-// 4% of the best depth on each.
+// them computed), and two CTAs fit on an SM: the depth is the one whose CTAs,
+// placed in launch order (the last chunk, whose planes may be fewer, comes last),
+// end first.  CTAs left over after full waves cost nearly a wave of their own:
+// alone on an SM a plane still takes 0.82 of its time beside another CTA.
+// Measured per launch: 32^3 137 us at a depth of 16 -> 31, 64^3 142 -> 53, 75^3
+// (FP64 state) 198 -> 129; against a rule that let a wave be 6% over: 100^3
+// (FP64 state; 1.05 -> 0.88 waves) 337 -> 260 us, 160^3 955 -> 698, 256^3 (FP32
+// state; 6.05 -> 6.92 waves) 1830 -> 1699.  The choice is within 4% of the best
+// depth on each of 32^3 to 320^3.
 int ctx_fp32_zchunk(const trg_ctx* c) {
 	int sms = 148;
 	cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->raw.device);
-	const long long tiles = (long long)((c->P.nx + 31) / 32) * ((c->P.ny + 7) / 8);
+	const long long tiles = (long long)((c->P.nx + 31) / 32) * ((c->P.ny + 7) / 8), slots = 2LL * sms;
 	int best = c->P.nz;
 	double best_cost = 1e300;
-	for (int chunks = 1; chunks <= c->P.nz; ++chunks) {
-		const int zc = (c->P.nz + chunks - 1) / chunks;
-		const long long ctas = tiles * ((c->P.nz + zc - 1) / zc);
-		const double cost = std::max(1.0, std::ceil((double)ctas / (2.0 * sms) - 0.06)) * (zc + 3.5);
+	for (int n = 1; n <= c->P.nz; ++n) {
+		const int zc = (c->P.nz + n - 1) / n, chunks = (c->P.nz + zc - 1) / zc;
+		const double full = zc + 3.5, last = c->P.nz - (long long)(chunks - 1) * zc + 3.5;
+		const long long ctas = tiles * (chunks - 1), waves = ctas / slots, over = ctas % slots;
+		const long long left = std::max(0LL, tiles - (slots - over));  // of the last chunk, beyond the wave
+		double cost = std::max((waves + (over > 0)) * full, waves * full + last);
+		if (left > 0)
+			cost = std::max(cost, waves * full + last +
+			                          (double)((left + slots - 1) / slots) * last * (left <= sms ? 0.82 : 1.0));
 		if (cost < best_cost) {
 			best_cost = cost;
 			best = zc;
