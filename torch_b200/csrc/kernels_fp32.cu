@@ -32,6 +32,16 @@
 // Pressure from total energy uses a compensated subtraction: the kinetic
 // energy is formed as a float pair with error-free products and sums, so that
 // E - KE loses no more than E's own rounding.
+//
+// Bound by instruction issue: two CTAs (16 warps) per SM issue in 60% of the
+// cycles, 2,180 instructions per cell's three faces, three slopes and update,
+// against 0.2 ms for the bytes of a 256^3 launch (FP32 state).  So branches with a
+// copy of a cell or a flux on either side are written as index or value
+// selects (one sequence of loads for the x, y and last faces, one flux per HLLC
+// solve, one branch per slope), and divisors that cannot be subnormal skip the
+// scaling for it.  Per launch: 256^3 FP32 state 2009 -> 1723 us, 256^3 HII region
+// (FP64 state) 2749 -> 2400 (both with the depth of the z chunks 37 -> 32, about
+// half of it), 75^3 HII region at the same depth 140 -> 128.
 #include <cuda.h>
 #include <cuda_runtime.h>
 
@@ -60,12 +70,30 @@ struct Scaled {
 		  Rg((float)(P.specificGasConstant * P.f32_rho0 / P.f32_p0)), X((float)P.X), gamma((float)P.gamma), nd(P.nd) {}
 };
 
-__device__ __forceinline__ float fminf_(float a, float b) { return (b < a) ? b : a; }
+// (b < a) ? b : a and (a < b) ? b : a with a constant b: a NaN in a stays one
+__device__ __forceinline__ float fminf_(float a, float b) {
+	float r;
+	asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+	return r;
+}
+__device__ __forceinline__ float fmaxf_(float a, float b) {
+	float r;
+	asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+	return r;
+}
 // Division and reciprocal of the FP32 form: the hardware approximation (one
 // reciprocal and one multiply, within 2 ulp for divisors of magnitude in
 // [2^-126, 2^126], which the scaled units keep every divisor of this file in).
 __device__ __forceinline__ float fdiv(float a, float b) { return __fdividef(a, b); }
 __device__ __forceinline__ float frcp(float b) { return __fdividef(1.0f, b); }
+// The same where b is 0 or of magnitude 2^-126 or more, whatever the state: no
+// scaling of subnormal divisors, which is most of a division's instructions.
+__device__ __forceinline__ float nrcp(float b) {
+	float r;
+	asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b));
+	return r;
+}
+__device__ __forceinline__ float ndiv(float a, float b) { return __fmul_rn(a, nrcp(b)); }
 // ... and the correctly rounded ones, kept in the radiation-hydro form (FP64
 // state, CR = true below) where the rounding noise of every hydro sub-step
 // feeds the long-run error against the FP64 form most: the reciprocal density
@@ -77,7 +105,6 @@ __device__ __forceinline__ float frcp(float b) { return __fdividef(1.0f, b); }
 __device__ __forceinline__ float pdiv(float a, float b) { return __fdiv_rn(a, b); }
 __device__ __forceinline__ float prcp(float b) { return __frcp_rn(b); }
 __device__ __forceinline__ float psqrt(float a) { return __fsqrt_rn(a); }
-__device__ __forceinline__ float fmaxf_(float a, float b) { return (a < b) ? b : a; }
 
 // Conserved-state storage of the FP32 kernels: float arrays hold the scaled
 // units directly; double arrays (the operator split's FP64 state) hold code
@@ -194,10 +221,6 @@ __device__ __forceinline__ bool fix_cons(const Scaled& P, float* u) {
 // left to the compiler), so that every call site computes a cell's slope and
 // face states identically: a face shared by two z chunks of the tiling gets
 // the same flux from both.
-__device__ __forceinline__ float albada(float a, float b, float thr) {
-	float ab = __fmul_rn(a, b);
-	return ab <= thr ? 0.f : fdiv(__fmul_rn(ab, __fadd_rn(a, b)), __fmaf_rn(a, a, __fmul_rn(b, b)));
-}
 __device__ __forceinline__ float minmod_(float a, float b) {
 	return (a * b > 0) ? (fabsf(a) < fabsf(b) ? a : b) : 0.f;
 }
@@ -219,7 +242,7 @@ __device__ __forceinline__ float limiter32(int kind, float a, float b, float thr
 		const float ab = __fmul_rn(a, b), t = __fmaf_rn(a, a, ab);
 		return (ab <= thr) ? 0.f : fdiv(__fmul_rn(__fmul_rn(1.5f, b), t), __fmaf_rn(b, b, t));
 	}
-	default: return albada(a, b, thr);
+	default: return 0.f;  // (albada: slope_of)
 	}
 }
 
@@ -233,6 +256,36 @@ struct LimThr {
 // QR(c1) = c1 + slope(c1) / 2 and QL(c2) = c2 - slope(c2) / 2.
 __device__ __forceinline__ Prim slope_of(int lim, const LimThr& th, const Prim& cm, const Prim& c, const Prim& cp) {
 	Prim s;
+	if (lim < 0 || lim > 5) {  // albada, its seven fields under one branch (below) instead of one each
+		const float dm[7] = {c.d - cm.d, c.p - cm.p, c.x - cm.x, c.a - cm.a, c.v[0] - cm.v[0], c.v[1] - cm.v[1], c.v[2] - cm.v[2]};
+		const float dp[7] = {cp.d - c.d, cp.p - c.p, cp.x - c.x, cp.a - c.a, cp.v[0] - c.v[0], cp.v[1] - c.v[1], cp.v[2] - c.v[2]};
+		const float thr[7] = {th.d, th.p, th.x, th.x, th.v, th.v, th.v};
+		float r[7];
+		bool flat = true;  // no slope in any field, as in gas at rest
+#pragma unroll
+		for (int i = 0; i < 7; ++i) {
+			r[i] = 0.f;
+			flat &= __fmul_rn(dm[i], dp[i]) <= thr[i];
+		}
+		if (!flat) {
+#pragma unroll
+			for (int i = 0; i < 7; ++i) {
+				const float ab = __fmul_rn(dm[i], dp[i]);
+				// (a subnormal a^2 + b^2 has a numerator that is 0)
+				const float den = fmaxf(__fmaf_rn(dm[i], dm[i], __fmul_rn(dp[i], dp[i])), 1.17549435e-38f);
+				const float v = ndiv(__fmul_rn(ab, __fadd_rn(dm[i], dp[i])), den);
+				r[i] = ab <= thr[i] ? 0.f : v;
+			}
+		}
+		s.d = r[0];
+		s.p = r[1];
+		s.x = r[2];
+		s.a = r[3];
+		s.v[0] = r[4];
+		s.v[1] = r[5];
+		s.v[2] = r[6];
+		return s;
+	}
 #define SLOPE(field, thr) s.field = limiter32(lim, c.field - cm.field, cp.field - c.field, thr);
 	SLOPE(d, th.d) SLOPE(p, th.p) SLOPE(x, th.x) SLOPE(a, th.x) SLOPE(v[0], th.v) SLOPE(v[1], th.v) SLOPE(v[2], th.v)
 #undef SLOPE
@@ -285,7 +338,7 @@ __device__ __forceinline__ void face_pre(const Prim& L, const Prim& R, float gam
 	cons_of(R, g1inv, f.UR);
 	f.sl = CR ? psqrt(L.d) : sqrtf(L.d);
 	f.sr = CR ? psqrt(R.d) : sqrtf(R.d);
-	f.inv = CR ? prcp(f.sl + f.sr) : frcp(f.sl + f.sr);
+	f.inv = CR ? prcp(f.sl + f.sr) : nrcp(f.sl + f.sr);
 	f.nu2 = 0.5f * f.sr * f.sl * f.inv * f.inv;
 	float aL2 = CR ? pdiv(gamma * L.p, L.d) : fdiv(gamma * L.p, L.d);
 	float aR2 = CR ? pdiv(gamma * R.p, R.d) : fdiv(gamma * R.p, R.d);
@@ -316,43 +369,48 @@ __device__ __forceinline__ void hll_n(const Prim& L, const Prim& R, const FacePr
 	flux_n(L, f.UL, n, unL, FL);
 	flux_n(R, f.UR, n, unR, FR);
 	speeds_n<CR>(f, unL, unR, SL, SR);
-	if (SR <= 0) {
-		for (int i = 0; i < 7; ++i) F[i] = FR[i];
-	} else if (SL >= 0) {
-		for (int i = 0; i < 7; ++i) F[i] = FL[i];
-	} else {
-		float inv = frcp(SR - SL);
-		for (int i = 0; i < 7; ++i) F[i] = (SR * FL[i] - SL * FR[i] + SL * SR * (f.UR[i] - f.UL[i])) * inv;
-	}
+	const float inv = nrcp(SR - SL);
+	for (int i = 0; i < 7; ++i) F[i] = (SR * FL[i] - SL * FR[i] + SL * SR * (f.UR[i] - f.UL[i])) * inv;
+	if (SR <= 0 || SL >= 0)
+		for (int i = 0; i < 7; ++i) F[i] = SR <= 0 ? FR[i] : FL[i];
 }
 
 template <bool CR>
 __device__ __forceinline__ void hllc_n(const Prim& L, const Prim& R, const FacePre& f, const float* n, float* F) {
-	float FL[7], FR[7], unL, unR, SL, SR;
-	flux_n(L, f.UL, n, unL, FL);
-	flux_n(R, f.UR, n, unR, FR);
+	const float unL = L.v[0] * n[0] + L.v[1] * n[1] + L.v[2] * n[2];
+	const float unR = R.v[0] * n[0] + R.v[1] * n[1] + R.v[2] * n[2];
+	float SL, SR;
 	speeds_n<CR>(f, unL, unR, SL, SR);
-	if (SL >= 0) {
-		for (int i = 0; i < 7; ++i) F[i] = FL[i];
-	} else if (SR <= 0) {
-		for (int i = 0; i < 7; ++i) F[i] = FR[i];
-	} else {
-		float mL = L.d * (SL - unL), mR = R.d * (SR - unR);
-		float Sc = fdiv(R.p - L.p + mL * unL - mR * unR, mL - mR);
-		bool left = Sc >= 0;
-		const Prim& K = left ? L : R;
-		const float* UK = left ? f.UL : f.UR;
-		const float* FK = left ? FL : FR;
-		float SK = left ? SL : SR, unK = left ? unL : unR;
-		float mK = K.d * (SK - unK);
-		float A = fdiv(mK, SK - Sc);
+	const float mL = L.d * (SL - unL), mR = R.d * (SR - unR);
+	const float Sc = fdiv(R.p - L.p + mL * unL - mR * unR, mL - mR);
+	// the side whose flux the face takes is chosen first and its flux formed once:
+	// selects instead of three branches with a copy of the flux in each
+	const bool pure = SL >= 0 || SR <= 0;
+	const bool left = SL >= 0 || (!(SR <= 0) && Sc >= 0);
+	Prim K;
+	K.d = left ? L.d : R.d;
+	K.p = left ? L.p : R.p;
+	K.x = left ? L.x : R.x;
+	K.a = left ? L.a : R.a;
+	for (int k = 0; k < 3; ++k) K.v[k] = left ? L.v[k] : R.v[k];
+	float UK[7];
+	for (int i = 0; i < 7; ++i) UK[i] = left ? f.UL[i] : f.UR[i];
+	const float SK = left ? SL : SR, unK = left ? unL : unR, mK = left ? mL : mR;
+	const float mflux = __fmul_rn(K.d, unK);
+	F[DEN] = mflux;
+	F[PRE] = __fmul_rn(UK[PRE] + K.p, unK);
+	F[HII] = __fmul_rn(mflux, K.x);
+	F[ADV] = __fmul_rn(mflux, K.a);
+	for (int k = 0; k < 3; ++k) F[VEL + k] = __fmaf_rn(mflux, K.v[k], __fmul_rn(K.p, n[k]));
+	if (!pure) {
+		const float A = fdiv(mK, SK - Sc);
 		float Us[7];
 		Us[DEN] = A;
 		Us[PRE] = A * (fdiv(UK[PRE], K.d) + (Sc - unK) * (Sc + fdiv(K.p, mK)));
 		Us[HII] = A * K.x;
 		Us[ADV] = A * K.a;
 		for (int k = 0; k < 3; ++k) Us[VEL + k] = A * (K.v[k] + (Sc - unK) * n[k]);
-		for (int i = 0; i < 7; ++i) F[i] = FK[i] + SK * (Us[i] - UK[i]);
+		for (int i = 0; i < 7; ++i) F[i] = F[i] + SK * (Us[i] - UK[i]);
 	}
 }
 
@@ -378,8 +436,8 @@ __device__ __forceinline__ void riemann32(int kind, const Prim& L, const Prim& R
 	float w1 = kind == RS_HLL ? 1.f : 0.f, w2 = kind == RS_HLLC ? 1.f : 0.f;
 	if (kind == RS_ROTATED) {
 		const float dv[3] = {R.v[0] - L.v[0], R.v[1] - L.v[1], R.v[2] - L.v[2]};
-		const float par = dv[0] * d[0] + dv[1] * d[1] + dv[2] * d[2];  // exact: one term is non-zero
-		const float perp[3] = {dv[0] - par * d[0], dv[1] - par * d[1], dv[2] - par * d[2]};  // exact
+		const float par = dim == 0 ? dv[0] : (dim == 1 ? dv[1] : dv[2]);
+		const float perp[3] = {dim == 0 ? 0.f : dv[0], dim == 1 ? 0.f : dv[1], dim == 2 ? 0.f : dv[2]};
 		const float pp = perp[0] * perp[0] + perp[1] * perp[1] + perp[2] * perp[2];
 		const float rr = par * par + pp;
 		if (rr < 1.0e-12f || par == 0.f) {  // |dv| < 1e-6, or dv normal to d: HLLC
@@ -388,24 +446,44 @@ __device__ __forceinline__ void riemann32(int kind, const Prim& L, const Prim& R
 			w1 = 1.f;
 		} else {
 			const float r = sqrtf(rr), s = sqrtf(pp);
-			const float inv_r = frcp(r);
+			const float inv_r = nrcp(r);
 			const float sg = par < 0 ? -1.f : 1.f;
 #pragma unroll
 			for (int k = 0; k < 3; ++k) n1[k] = sg * dv[k] * inv_r;
 			w1 = fabsf(par) * inv_r;
 			w2 = s * inv_r;
-			const float k2 = fdiv(par * inv_r, s);
+			const float k2 = ndiv(__fmul_rn(par, inv_r), s);
 #pragma unroll
-			for (int k = 0; k < 3; ++k) n2[k] = w2 * d[k] - k2 * perp[k];
+			for (int k = 0; k < 3; ++k) n2[k] = dim == k ? w2 : -__fmul_rn(k2, perp[k]);
 		}
 	}
-	float F1[7], F2[7];
+	// F = w1 F1 + w2 F2, rounded the same in both orders of evaluation: with the
+	// HLLC part formed first and scaled in place fewer registers are live (FP32
+	// state, 1772 -> 1726 us per 256^3 launch); with the correctly rounded
+	// operations that order spills (2407 against 2494 us)
+	if constexpr (CR) {
+		float F2[7];
 #pragma unroll
-	for (int i = 0; i < 7; ++i) F1[i] = F2[i] = 0.f;
-	if (w1 != 0.f) hll_n<CR>(L, R, f, n1, F1);
-	if (w2 != 0.f) hllc_n<CR>(L, R, f, n2, F2);
+		for (int i = 0; i < 7; ++i) F[i] = F2[i] = 0.f;
+		if (w1 != 0.f) hll_n<CR>(L, R, f, n1, F);
+		if (w2 != 0.f) hllc_n<CR>(L, R, f, n2, F2);
 #pragma unroll
-	for (int i = 0; i < 7; ++i) F[i] = w1 * F1[i] + w2 * F2[i];
+		for (int i = 0; i < 7; ++i) F[i] = __fmaf_rn(w1, F[i], __fmul_rn(w2, F2[i]));
+	} else {
+#pragma unroll
+		for (int i = 0; i < 7; ++i) F[i] = 0.f;
+		if (w2 != 0.f) {
+			hllc_n<CR>(L, R, f, n2, F);
+#pragma unroll
+			for (int i = 0; i < 7; ++i) F[i] = __fmul_rn(w2, F[i]);
+		}
+		if (w1 != 0.f) {
+			float F1[7];
+			hll_n<CR>(L, R, f, n1, F1);
+#pragma unroll
+			for (int i = 0; i < 7; ++i) F[i] = __fmaf_rn(w1, F1[i], F[i]);
+		}
+	}
 }
 
 // A Prim, or a flux, in shared memory as two 16-byte halves kept in two
@@ -765,17 +843,13 @@ __device__ __forceinline__ void hydro_stage_body(const Params& P, const State& S
 	constexpr bool CR = sizeof(TS) == sizeof(double);  // the radiation-hydro form's correctly rounded operations
 	SmemQ& s = *reinterpret_cast<SmemQ*>(smem_raw);
 	float4* v8 = reinterpret_cast<float4*>(smem_raw + sizeof(SmemQ));
-	const V8 Fx{v8, v8 + N_FX};                      // [BY][BX + 1] x-face fluxes
-	v8 += 2 * N_FX;
-	const V8 Fy{v8, v8 + N_FY};                      // [BY + 1][BX] y-face fluxes
-	v8 += 2 * N_FY;
-	const V8 Sx{v8, v8 + N_S};                       // [BY * BX] x slopes of the tile
-	v8 += 2 * N_S;
-	const V8 Sy{v8, v8 + N_S};                       // [BY * BX] y slopes of the tile
-	v8 += 2 * N_S;
-	const V8 Ex{v8, v8 + N_EX};                      // [2 * BY] x slopes of cells x0 - 1, x0 + BX
-	v8 += 2 * N_EX;
-	const V8 Ey{v8, v8 + N_EY};                      // [2 * BX] y slopes of cells y0 - 1, y0 + BY
+	// face fluxes: x faces [BY][BX + 1], then y faces [BY + 1][BX]
+	const V8 FL{v8, v8 + N_FX + N_FY};
+	v8 += 2 * (N_FX + N_FY);
+	// slopes: x and y of the tile's cells, x of the cells x0 - 1 and x0 + BX, y
+	// of the cells y0 - 1 and y0 + BY
+	constexpr int I_SY = N_S, I_EX = 2 * N_S, I_EY = I_EX + N_EX;
+	const V8 SL{v8, v8 + I_EY + N_EY};
 	TS* raw = reinterpret_cast<TS*>(smem_raw + hydro_stage_raw_offset());  // [7][SY * SX] next plane, staged
 	uint64_t* tbar = reinterpret_cast<uint64_t*>(smem_raw + hydro_stage_raw_offset() + sizeof(double) * 7 * SX * SY);
 	const int tx = threadIdx.x % BX, ty = threadIdx.x / BX;
@@ -808,7 +882,8 @@ __device__ __forceinline__ void hydro_stage_body(const Params& P, const State& S
 	                           : (te < BX + BY && x0 + BX <= P.nx && y0 + te - BX < P.ny);
 	// edge slopes (cells just outside the tile): the last 80 threads
 	const int ts = (int)threadIdx.x - (BX * BY - 2 * (BX + BY));
-	double tmin = 1.0e308;
+	double inv_max = 0;  // the CFL limit is half the reciprocal of the largest 1/t
+	const double v_dx = STAGE == 2 ? P.f32_v0 / P.dx[0] : 0.0;
 	bool bad = false;
 
 	// geometry of this thread's cell column: cartesian factors are uniform
@@ -884,16 +959,16 @@ __device__ __forceinline__ void hydro_stage_body(const Params& P, const State& S
 		}
 		if (rec && plane) {
 			const Prim qc = get(s, sc, ly, lx);
-			Sx.put(threadIdx.x, slope_of(lim, th, get(s, sc, ly, lx - 1), qc, get(s, sc, ly, lx + 1)));
+			SL.put(threadIdx.x, slope_of(lim, th, get(s, sc, ly, lx - 1), qc, get(s, sc, ly, lx + 1)));
 			if (nd > 1)
-				Sy.put(threadIdx.x, slope_of(lim, th, get(s, sc, ly - 1, lx), qc, get(s, sc, ly + 1, lx)));
+				SL.put(I_SY + threadIdx.x, slope_of(lim, th, get(s, sc, ly - 1, lx), qc, get(s, sc, ly + 1, lx)));
 			if (ts >= 0 && ts < 2 * BY) {
 				const int e = ts / BY, r = ts - e * BY, ex = e ? HALO + BX : HALO - 1;
-				Ex.put(ts,
+				SL.put(I_EX + ts,
 				     slope_of(lim, th, get(s, sc, r + HALO, ex - 1), get(s, sc, r + HALO, ex), get(s, sc, r + HALO, ex + 1)));
 			} else if (ts >= 2 * BY && nd > 1) {
 				const int u = ts - 2 * BY, e = u / BX, col = u - e * BX, ey = e ? HALO + BY : HALO - 1;
-				Ey.put(u,
+				SL.put(I_EY + u,
 				     slope_of(lim, th, get(s, sc, ey - 1, col + HALO), get(s, sc, ey, col + HALO), get(s, sc, ey + 1, col + HALO)));
 			}
 		}
@@ -906,61 +981,35 @@ __device__ __forceinline__ void hydro_stage_body(const Params& P, const State& S
 		const int nk = te < BX + BY ? 3 : 2;  // only threads 0 .. BX + BY - 1 take a last face
 #pragma unroll 1
 		for (int k = 0; k < nk; ++k) {
-			Prim ql, qr, sl = zero, sr = zero;
-			int dim;
-			bool ok;
-			V8 dst;
-			int di;
-			if (k == 0) {  // x face gx - 1/2, between cells lx - 1 and lx of row ly
-				ok = fx_ok && plane;
-				dim = 0;
-				ql = get(s, sc, ly, lx - 1);
-				qr = get(s, sc, ly, lx);
-				if (rec && ok) {
-					sl = tx > 0 ? Sx.get(threadIdx.x - 1) : Ex.get(ty);
-					sr = Sx.get(threadIdx.x);
-				}
-				dst = Fx;
-				di = ty * (BX + 1) + tx;
-			} else if (k == 1) {  // y face gy - 1/2, between rows ly - 1 and ly of column lx
-				ok = fy_ok && plane;
-				dim = 1;
-				ql = get(s, sc, ly - 1, lx);
-				qr = get(s, sc, ly, lx);
-				if (rec && ok) {
-					sl = ty > 0 ? Sy.get(threadIdx.x - BX) : Ey.get(tx);
-					sr = Sy.get(threadIdx.x);
-				}
-				dst = Fy;
-				di = ty * BX + tx;
-			} else if (te < BX) {  // y face y0 + BY - 1/2 of column te
-				ok = fe_ok && plane;
-				dim = 1;
-				ql = get(s, sc, HALO + BY - 1, te + HALO);
-				qr = get(s, sc, HALO + BY, te + HALO);
-				if (rec && ok) {
-					sl = Sy.get((BY - 1) * BX + te);
-					sr = Ey.get(BX + te);
-				}
-				dst = Fy;
-				di = BY * BX + te;
-			} else {  // x face x0 + BX - 1/2 of row te - BX
-				ok = fe_ok && plane;
-				dim = 0;
-				const int r = min(te - BX, BY - 1);
-				ql = get(s, sc, r + HALO, HALO + BX - 1);
-				qr = get(s, sc, r + HALO, HALO + BX);
-				if (rec && ok) {
-					sl = Sx.get(r * BX + BX - 1);
-					sr = Ex.get(BY + r);
-				}
-				dst = Fx;
-				di = r * (BX + 1) + BX;
+			// cells and slopes on either side of the face and its place, as indices:
+			// one sequence of loads for all three kinds
+			int qi, di, sl, sr, step;
+			bool ok = plane;
+			const bool x_face = k == 0 || (k == 2 && te >= BX);
+			if (k < 2) {  // x face gx - 1/2 or y face gy - 1/2, below the cell
+				ok &= x_face ? fx_ok : fy_ok;
+				qi = ly * SX + lx;
+				sr = x_face ? (int)threadIdx.x : I_SY + (int)threadIdx.x;
+				sl = x_face ? (tx > 0 ? sr - 1 : I_EX + ty) : (ty > 0 ? sr - BX : I_EY + tx);
+				di = x_face ? ty * (BX + 1) + tx : N_FX + ty * BX + tx;
+			} else {  // y face y0 + BY - 1/2 of column te, x face x0 + BX - 1/2 of row te - BX
+				ok &= fe_ok;
+				const int r = te - BX;
+				qi = x_face ? (r + HALO) * SX + HALO + BX : (HALO + BY) * SX + te + HALO;
+				sl = x_face ? r * BX + BX - 1 : I_SY + (BY - 1) * BX + te;
+				sr = x_face ? I_EX + BY + r : I_EY + BX + te;
+				di = x_face ? r * (BX + 1) + BX : N_FX + BY * BX + te;
 			}
+			step = x_face ? 1 : SX;
 			if (!ok) continue;
+			Prim ql = s.ring(sc).get(qi - step), qr = s.ring(sc).get(qi);
+			if (rec) {
+				ql = face_left(ql, SL.get(sl));
+				qr = face_right(qr, SL.get(sr));
+			}
 			float f[7];
-			face_flux<RS, CR>(rs_rt, rec ? face_left(ql, sl) : ql, rec ? face_right(qr, sr) : qr, dim, gamma, f);
-			dst.put_f(di, f);
+			face_flux<RS, CR>(rs_rt, ql, qr, x_face ? 0 : 1, gamma, f);
+			FL.put_f(di, f);
 		}
 		float fz[7];  // flux through this column's face z + 1/2
 		if (nd > 2) {
@@ -983,13 +1032,13 @@ __device__ __forceinline__ void hydro_stage_body(const Params& P, const State& S
 		if (active && plane) {
 			const long long id = gx + (long long)P.nx * (gy + (long long)P.ny * z);
 			float udot[7], fl[7], fr[7];
-			Fx.get_f(ty * (BX + 1) + tx, fl);
-			Fx.get_f(ty * (BX + 1) + tx + 1, fr);
+			FL.get_f(ty * (BX + 1) + tx, fl);
+			FL.get_f(ty * (BX + 1) + tx + 1, fr);
 #pragma unroll
 			for (int i = 0; i < 7; ++i) udot[i] = axl * fl[i] - axr * fr[i];
 			if (nd > 1) {
-				Fy.get_f(ty * BX + tx, fl);
-				Fy.get_f((ty + 1) * BX + tx, fr);
+				FL.get_f(N_FX + ty * BX + tx, fl);
+				FL.get_f(N_FX + (ty + 1) * BX + tx, fr);
 #pragma unroll
 				for (int i = 0; i < 7; ++i) udot[i] += ayl * fl[i] - ayr * fr[i];
 			}
@@ -1050,9 +1099,9 @@ __device__ __forceinline__ void hydro_stage_body(const Params& P, const State& S
 				double inv_t = 0;
 #pragma unroll
 				for (int k = 0; k < 3; ++k)
-					if (k < nd) inv_t += (fabs((double)q.v[k]) + ss) * P.f32_v0 / P.dx[k];
+					if (k < nd) inv_t += (fabs((double)q.v[k]) + ss) * v_dx;
 				if (inv_t == 0) inv_t = 1.0 / P.dt_max;
-				tmin = dmin_(tmin, 0.5 / inv_t);
+				inv_max = inv_t > inv_max ? inv_t : inv_max;
 			}
 		}
 		if (nd > 2) {
@@ -1068,6 +1117,7 @@ __device__ __forceinline__ void hydro_stage_body(const Params& P, const State& S
 	if (bad) atomicOr(S.err, ERRB_NAN);
 	if (tma_late) atomicOr(S.err, ERRB_ASYNC);
 	if (STAGE == 2) {
+		double tmin = inv_max > 0 ? 0.5 / inv_max : 1.0e308;
 		for (int o = 16; o > 0; o >>= 1) tmin = dmin_(tmin, __shfl_down_sync(0xffffffffu, tmin, o));
 		if ((threadIdx.x & 31) == 0) {
 			unsigned long long* slots = reinterpret_cast<unsigned long long*>(S.scal + 2);
