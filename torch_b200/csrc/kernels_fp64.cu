@@ -354,17 +354,11 @@ __device__ __forceinline__ void neighbours(const Params& P, const SweepCell& c, 
 		}
 	}
 	const double x0 = pick3(c.x[0], c.x[1], c.x[2], r0), x1 = pick3(c.x[0], c.x[1], c.x[2], r1);
-#ifdef TRG_FAST_MATH
-	// one division; a neighbour level with the cell where the axes tie has a
-	// weight of exactly 0 (it belongs to the cell's own shell), which the
-	// rounded reciprocal would not give
-	const double inv2 = (double)s2 / (double)e2;
-	const double ic0 = x0 - 0.5 * (abs(e0) == abs(e2) ? (double)s0 : (double)e0 * inv2);
-	const double ic1 = x1 - 0.5 * (abs(e1) == abs(e2) ? (double)s1 : (double)e1 * inv2);
-#else
-	const double ic0 = x0 - 0.5 * ((double)(s2 * e0) / (double)e2);
-	const double ic1 = x1 - 0.5 * ((double)(s2 * e1) / (double)e2);
-#endif
+	// (both quotients correctly rounded: +-1 exactly, and with it a weight of
+	// exactly 0, where the axes tie and the neighbour lies in the cell's own shell)
+	Recip r;
+	r.set((double)e2);
+	const double ic0 = x0 - 0.5 * r.div((double)(s2 * e0)), ic1 = x1 - 0.5 * r.div((double)(s2 * e1));
 	const double delta0 = fabs(2.0 * ic0 - 2.0 * x0 + s0);
 	const double delta1 = fabs(2.0 * ic1 - 2.0 * x1 + s1);
 	const bool far0 = abs(e0) >= 2, far1 = abs(e1) >= 2, far2 = abs(e2) >= 2;  // |d| > 0.9
@@ -1233,7 +1227,7 @@ __global__ void __launch_bounds__(256) k_rad_update_fp64(Params P, State S, doub
 	b_rad_update_fp64(P, S, id, h, mode);
 }
 
-// The radiation and thermal updates of the FP32 form (NEQ coupling), where U has
+// The radiation and thermal updates of the FP32 form's 3-D grids (NEQ coupling), where U has
 // come out of an update before (every field within its floors) and Q holds its
 // primitives: they write what a sub-step changes.  A cell radiation leaves
 // alone (no heating, x_HII and ADV as U has them: the neutral gas beyond the
@@ -1278,13 +1272,6 @@ __device__ __forceinline__ void b_rad_update_lean(const Params& P, const State& 
 }
 __global__ void __launch_bounds__(256) k_rad_update_lean(Params P, State S, double h) {
 	grid_begin();
-	if (TRG_BATCHED && P.batch) {
-		const BatchTable& B = *P.batch;
-		const int g = batch_slot(B.cell_off, B.G, blockIdx.x * (long long)blockDim.x);
-		const long long lid = blockIdx.x * (long long)blockDim.x + threadIdx.x - B.cell_off[g];
-		if (lid < B.P[g].N) b_rad_update_lean(B.P[g], B.S[g], lid, h);
-		return;
-	}
 	const long long id = blockIdx.x * (long long)blockDim.x + threadIdx.x;
 	if (id < P.N) b_rad_update_lean(P, S, id, h);
 }
@@ -1755,13 +1742,6 @@ __device__ __forceinline__ void b_thermo_lean(const Params& P, const State& S, l
 }
 __global__ void __launch_bounds__(256) k_thermo_lean(Params P, State S, double h, int update_only) {
 	grid_begin();
-	if (TRG_BATCHED && P.batch) {
-		const BatchTable& B = *P.batch;
-		const int g = batch_slot(B.cell_off, B.G, blockIdx.x * (long long)blockDim.x);
-		const long long lid = blockIdx.x * (long long)blockDim.x + threadIdx.x - B.cell_off[g];
-		if (lid < B.P[g].N) b_thermo_lean(B.P[g], B.S[g], lid, h, update_only);
-		return;
-	}
 	const long long id = blockIdx.x * (long long)blockDim.x + threadIdx.x;
 	if (id < P.N) b_thermo_lean(P, S, id, h, update_only);
 }
