@@ -32,7 +32,12 @@ def wrong():
     subprocess.run(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-o", so, src], check=True)
     fn = C.CDLL(so).wrong
     fn.restype, fn.argtypes = C.c_long, [C.c_uint, C.c_void_p, C.c_long]
-    return lambda d, n: fn(d, np.ascontiguousarray(n, dtype=np.uint32).ctypes.data, len(n))
+
+    def count(d, n):
+        a = np.ascontiguousarray(n, dtype=np.uint32)  # held over the call
+        return fn(d, a.ctypes.data, len(a))
+
+    return count
 
 
 def indices(d, rng):
