@@ -72,6 +72,10 @@ struct trg_ctx {
 	// FP32 form with radiation/cooling: U has come out of an update since the
 	// host last set it, so every field is within its floors
 	bool u_fixed = false;
+	// heating rates (T_HEAT) are in place for the next thermal sub-step, and
+	// another sub-step has run since, so that cells now below the HII switch may
+	// hold one
+	bool rates_set = false, heat_below = false;
 	// the column densities of the thermodynamics depend on the density alone,
 	// which only hydro sub-steps change: a second sweep with no hydro sub-step
 	// since the last one would recompute the same values and is skipped
@@ -432,6 +436,7 @@ void thermo_pre(trg_ctx* c) {
 		c->colden_valid = true;
 	}
 	LAUNCH(KF(k_thermo_rates_fp64), c->P.N, 256, c->P, c->S);
+	c->rates_set = true;
 }
 
 void rad_pre(trg_ctx* c) { LAUNCH(KF(k_rad_heating_fp64), c->P.N, 256, c->P, c->S); }
@@ -669,16 +674,18 @@ void sub_step(trg_ctx* c, double h, bool hasCalculatedHeatFlux, int comp, bool l
 		// (with the work queue, and where the heating terms are kept, the
 		// sub-cycles run in a pass of their own)
 		if (lean && c->P.thermo_subcycling && !c->S.thq && !c->S.H) {
-			LAUNCH(KF(k_thermo_lean), c->P.N, 256, c->P, c->S, h, 0);
+			LAUNCH(KF(k_thermo_lean), c->P.N, 256, c->P, c->S, h, 0, c->heat_below);
 		} else {
 			thermo_integrate(c, h);
-			if (lean) LAUNCH(KF(k_thermo_lean), c->P.N, 256, c->P, c->S, h, 1);
+			if (lean) LAUNCH(KF(k_thermo_lean), c->P.N, 256, c->P, c->S, h, 1, c->heat_below);
 			else LAUNCH(KF(k_thermo_update_fp64), c->P.N, 256, c->P, c->S, h, with_q ? 2 : 0);
 		}
 		c->q_fresh = with_q;
 		break;
 	}
 	c->u_fixed = c->mixed;
+	c->rates_set = c->rates_set && comp != COMP_THERMO;
+	c->heat_below = c->rates_set;
 }
 
 void hydro_step(trg_ctx* c) {
@@ -1435,6 +1442,7 @@ int trg_checkpoint_load(trg_ctx* c, const void* buf, long long bytes) {
 	CUDA_TRY(cudaMemset(c->S.UDOT, 0, 7 * N * sizeof(double)));
 	c->q_fresh = h.q_fresh != 0;
 	c->colden_valid = false;
+	c->rates_set = c->heat_below = true;  // (as far as the blob tells)
 	c->prologue_colden = false;  // the restored T is the saved run's
 	c->steps = h.steps;
 	c->first_time = h.first_time;

@@ -1711,17 +1711,28 @@ __global__ void __launch_bounds__(256) k_thermo_update_fp64(Params P, State S, d
 // the update alone from the rate that sub-cycles have left in T_RATE (the FP32
 // form, see k_rad_update_lean): cells below the HII switch, whose rates the
 // rate pass has set to 0, and wind cells are left alone (8 bytes read); the
-// others change their pressure and energy only.
+// others change their pressure and energy only.  clear_heat: another sub-step
+// may have carried cells below the switch since a rate pass, and these still
+// hold their heating rate of before (8 bytes more); like every cell outside
+// the wind they end the sub-step with none.  (Asked for in one of a step's two
+// thermal sub-steps or none; always asked for, the 256^3 step would be 1% longer.)
+__device__ __forceinline__ bool is_wind(const Params& P, long long id) {
+	int ijk[3];
+	double xc[3];
+	cell_ijk(P, id, ijk);
+	cell_xc(P, ijk, xc);
+	return is_wind(P, id, ijk, xc);
+}
 __device__ __forceinline__ void b_thermo_lean(const Params& P, const State& S, long long id, double h,
-                                              int update_only) {
-	if (FLD(S.Q, ADV, id) < P.thermo_hii_switch) return;
+                                              int update_only, int clear_heat) {
+	const double adv = FLD(S.Q, ADV, id), heat = clear_heat ? TFLD(S.T, T_HEAT, id) : 0.0;
+	if (adv < P.thermo_hii_switch) {
+		if (heat != 0 && !is_wind(P, id)) TFLD(S.T, T_HEAT, id) = 0;
+		return;
+	}
 	double rate;
 	if (update_only) {
-		int ijk[3];
-		double xc[3];
-		cell_ijk(P, id, ijk);
-		cell_xc(P, ijk, xc);
-		if (is_wind(P, id, ijk, xc)) return;
+		if (is_wind(P, id)) return;
 		rate = TFLD(S.T, T_RATE, id);
 	} else {
 		ThermoCell c;
@@ -1740,10 +1751,10 @@ __device__ __forceinline__ void b_thermo_lean(const Params& P, const State& S, l
 	TFLD(S.T, T_RATE, id) = 0;
 	TFLD(S.T, T_HEAT, id) = 0;
 }
-__global__ void __launch_bounds__(256) k_thermo_lean(Params P, State S, double h, int update_only) {
+__global__ void __launch_bounds__(256) k_thermo_lean(Params P, State S, double h, int update_only, int clear_heat) {
 	grid_begin();
 	const long long id = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-	if (id < P.N) b_thermo_lean(P, S, id, h, update_only);
+	if (id < P.N) b_thermo_lean(P, S, id, h, update_only, clear_heat);
 }
 
 // Thermodynamics::fillHeatingArrays (Thermodynamics.cpp:419-461) after its

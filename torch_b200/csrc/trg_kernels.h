@@ -45,7 +45,7 @@
 	__global__ void k_thq_drain(Params P, State S, double h); \
 	__global__ void k_thermo_update_fp64(Params P, State S, double h, int mode); \
 	__global__ void k_rad_update_lean(Params P, State S, double h); \
-	__global__ void k_thermo_lean(Params P, State S, double h, int update_only); \
+	__global__ void k_thermo_lean(Params P, State S, double h, int update_only, int clear_heat); \
 	__global__ void k_heating_arrays_fp64(Params P, State S); \
 	__global__ void k_fb_flags(Params P, State S, double contrast); \
 	__global__ void k_fb_faces(Params P, State S); \
