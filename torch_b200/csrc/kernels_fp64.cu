@@ -357,8 +357,8 @@ __device__ __forceinline__ void neighbours(const Params& P, const SweepCell& c, 
 	// (both quotients correctly rounded: +-1 exactly, and with it a weight of
 	// exactly 0, where the axes tie and the neighbour lies in the cell's own shell)
 	Recip r;
-	r.set((double)e2);
-	const double ic0 = x0 - 0.5 * r.div((double)(s2 * e0)), ic1 = x1 - 0.5 * r.div((double)(s2 * e1));
+	r.set((double)abs(e2));
+	const double ic0 = x0 - 0.5 * r.div((double)e0), ic1 = x1 - 0.5 * r.div((double)e1);
 	const double delta0 = fabs(2.0 * ic0 - 2.0 * x0 + s0);
 	const double delta1 = fabs(2.0 * ic1 - 2.0 * x1 + s1);
 	const bool far0 = abs(e0) >= 2, far1 = abs(e1) >= 2, far2 = abs(e2) >= 2;  // |d| > 0.9

@@ -49,22 +49,24 @@ __device__ __forceinline__ void grid_begin() {
 __device__ __forceinline__ double smin(double a, double b) { return (b < a) ? b : a; }
 __device__ __forceinline__ double smax(double a, double b) { return (a < b) ? b : a; }
 
-// Division by one divisor: a reciprocal by Newton's iteration, then a / b by
-// two corrections with exact remainders (P. Markstein, "Computation of
+// Division by one positive divisor: a reciprocal by Newton's iteration, then
+// a / b by two corrections with exact remainders (P. Markstein, "Computation of
 // elementary functions on the IBM RISC System/6000 processor", IBM J. R&D 34,
 // 1990): with y the correctly rounded reciprocal, which its last iteration
 // gives unless b's significand is all ones, and a quotient within one ulp,
-// fma(remainder, y, quotient) is a / b rounded to nearest.  Operands outside
-// 2^-500 .. 2^500 (where a remainder or a quotient could leave the normal
-// range) and such divisors take the built-in division.  It has no branch where
+// quotient + remainder y in one rounding is a / b rounded to nearest.  The
+// remainder is formed as b q - a, whose exact 0 is +0 and adds as -0: a zero
+// numerator keeps its sign.  Divisors and numerators outside 2^-500 .. 2^500
+// (where a remainder or a quotient could leave the normal range), negative
+// divisors and those significands take the built-in division.  It has no branch where
 // several quotients are tested together (takes), so that they overlap, and
 // costs five operations per quotient once the reciprocal is there; the built-in
 // one is a serial 112 cycles each, and more where the numerator is 0.
 struct Recip {
 	double b, y;
 	bool ok;
-	__device__ __forceinline__ static bool mid(double v) {  // 2^-500 <= |v| < 2^500
-		return (unsigned)(__double2hiint(v) & 0x7fffffff) - 0x20b00000u < 0x3e800000u;
+	__device__ __forceinline__ static bool mid(double v) {  // 2^-500 <= v < 2^500
+		return (unsigned)__double2hiint(v) - 0x20b00000u < 0x3e800000u;
 	}
 	__device__ __forceinline__ void set(double divisor) {
 		b = divisor;
@@ -76,10 +78,10 @@ struct Recip {
 	}
 	__device__ __forceinline__ double quotient(double a) const {
 		double q = a * y;
-		q = fma(fma(-b, q, a), y, q);
-		return fma(fma(-b, q, a), y, q);
+		q = fma(fma(b, q, -a), -y, q);
+		return fma(fma(b, q, -a), -y, q);
 	}
-	__device__ __forceinline__ bool takes(double a) const { return ok && (mid(a) || a == 0.0); }
+	__device__ __forceinline__ bool takes(double a) const { return ok && (mid(fabs(a)) || a == 0.0); }
 	__device__ __forceinline__ double div(double a) const { return takes(a) ? quotient(a) : a / b; }
 };
 
