@@ -1,0 +1,97 @@
+"""What the library launches and reports, on a CUDA runtime that runs nothing
+(fake_gpu)."""
+import dataclasses
+
+import numpy as np
+import pytest
+
+import fake_gpu
+import known_answers
+import torch_b200
+from torch_b200 import workloads
+
+FP64, FP32 = torch_b200.PRECISION_FP64, torch_b200.PRECISION_FP32
+
+
+@pytest.fixture
+def gpu():
+    with fake_gpu.fake_gpu() as g:
+        yield g
+
+
+def blister(nx=40, ny=53, wind=0):
+    tp, ic = workloads.blister((nx, ny, 1))
+    return dataclasses.replace(tp, windCellRadius=wind, massLossRate=tp.massLossRate if wind else 0.0), ic
+
+
+# --------------------------------------------------------- refused launches
+CASES = {
+    "spitzer_1d": (lambda: known_answers.spitzer_case(60, 6.0), FP64),
+    "blister_fp64": (blister, FP64),
+    "blister_fp32": (blister, FP32),
+    "hii_fp32": (lambda: workloads.hii_region(n=24, seed=1), FP32),
+    "sedov_fp64": (lambda: workloads.sedov(n=12), FP64),
+    "sedov_fp32": (lambda: workloads.sedov(n=12), FP32),
+}
+
+
+def kernels(gpu):
+    return sorted({l.name for l in gpu.launches()})
+
+
+@pytest.mark.parametrize("case", sorted(CASES))
+def test_refused_launches_are_reported(gpu, case):
+    """Whichever kernel of a run the runtime refuses to launch, in a captured
+    sweep or not: the call that needs it fails."""
+    make, form = CASES[case]
+    tp, ic = make()
+    t = torch_b200.Torch(tp, ic, precision=form)
+    created = kernels(gpu)
+    gpu.reset()
+    t.run_steps(6)
+    stepped = kernels(gpu)
+    t.close()
+    assert len(stepped) > 2
+    for name in created:
+        gpu.reset()
+        gpu.refuse(name)
+        with pytest.raises(torch_b200.TrgError):
+            torch_b200.Torch(tp, ic, precision=form)
+        assert gpu.counts()["refused"], name
+    for name in stepped:
+        gpu.reset()
+        t = torch_b200.Torch(tp, ic, precision=form)
+        gpu.refuse(name)
+        with pytest.raises(torch_b200.TrgError):
+            t.run_steps(6)
+        assert gpu.counts()["refused"], name
+        gpu.refuse("")
+        t.run_steps(2)  # reported once
+        t.close()
+
+
+@pytest.mark.parametrize("form", [FP64, FP32])
+def test_refused_launches_of_a_batch_are_reported(gpu, form):
+    def grids():
+        return [torch_b200.Torch(*blister(nx, ny), precision=form) for nx, ny in ((20, 33), (61, 17))]
+
+    g = grids()
+    b = torch_b200.Batch(g)
+    b.run_steps(2, g[0].dt_max)  # the first steps are not captured
+    gpu.reset()
+    b.run_steps(6, g[0].dt_max)
+    # (the column-density sweep has a graph of its own from the first steps, which takes over)
+    names = [n for n in kernels(gpu) if "colden" not in n]
+    assert gpu.counts()["graphs"] > 0
+    b.close()
+    for name in names:
+        g = grids()
+        b = torch_b200.Batch(g)
+        b.run_steps(2, g[0].dt_max)
+        gpu.reset()
+        gpu.refuse(name)
+        with pytest.raises(torch_b200.TrgError):
+            b.run_steps(6, g[0].dt_max)
+        assert gpu.counts()["refused"], name
+        gpu.refuse("")
+        b.close()

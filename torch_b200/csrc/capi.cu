@@ -147,6 +147,7 @@ struct trg_ctx {
 	long long cons_cap = 0;
 	bool cons_on = false;
 	std::string err;
+	cudaError_t launch_err = cudaSuccess;  // of launches before a capture, not reported yet
 	// optional per-launch CUDA-event timing
 	bool profiling = false;
 	struct Rec { const char* name; cudaEvent_t a, b; };
@@ -169,6 +170,21 @@ int set_error(trg_ctx* c, int code, const std::string& msg) {
 			return set_error(c, e_ == cudaErrorMemoryAllocation ? TRG_ERR_OOM : TRG_ERR_CUDA,         \
 			                 std::string(#call) + ": " + cudaGetErrorString(e_));                         \
 	} while (0)
+
+// The calling thread's launch errors so far, kept for the next report: a capture
+// that follows is judged by its own.
+void keep_launch_error(trg_ctx* c) {
+	const cudaError_t e = cudaGetLastError();
+	if (c->launch_err == cudaSuccess) c->launch_err = e;
+}
+int report_launch_error(trg_ctx* c) {
+	keep_launch_error(c);
+	const cudaError_t e = c->launch_err;
+	c->launch_err = cudaSuccess;
+	if (e == cudaSuccess) return TRG_OK;
+	return set_error(c, e == cudaErrorMemoryAllocation ? TRG_ERR_OOM : TRG_ERR_CUDA,
+	                 std::string("kernel launch: ") + cudaGetErrorString(e));
+}
 
 template <typename T>
 int dalloc(trg_ctx* c, T** p, size_t count) {
@@ -386,7 +402,9 @@ void colden_sweep_direct(trg_ctx* c) {
 	}
 }
 
-// Captures `body` (kernel launches on c->stream) into an executable graph.
+// Captures `body` (kernel launches on c->stream) into an executable graph.  A
+// refused launch can leave the capture valid, with a graph that lacks it: that
+// graph is dropped, and the launches that take its place report the refusal.
 template <typename F>
 cudaGraphExec_t capture_graph(trg_ctx* c, F body, long long& nodes) {
 	bool prof = c->profiling;
@@ -394,6 +412,7 @@ cudaGraphExec_t capture_graph(trg_ctx* c, F body, long long& nodes) {
 	long long before = c->launches;
 	cudaGraph_t g = nullptr;
 	cudaGraphExec_t ge = nullptr;
+	keep_launch_error(c);
 	if (cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
 		body();
 		if (cudaStreamEndCapture(c->stream, &g) == cudaSuccess && g) {
@@ -404,7 +423,10 @@ cudaGraphExec_t capture_graph(trg_ctx* c, F body, long long& nodes) {
 	nodes = c->launches - before;
 	c->launches = before;
 	c->profiling = prof;
-	cudaGetLastError();
+	if (cudaGetLastError() != cudaSuccess && ge) {
+		cudaGraphExecDestroy(ge);
+		ge = nullptr;
+	}
 	return ge;
 }
 
@@ -834,7 +856,7 @@ void enqueue_full_step(trg_ctx* c, double dt_next) {
 }
 
 int check_device_error(trg_ctx* c) {
-	CUDA_TRY(cudaGetLastError());
+	if (int rc = report_launch_error(c)) return rc;
 	unsigned e = 0;
 	CUDA_TRY(cudaMemcpyAsync(&e, c->S.err, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
 	CUDA_TRY(cudaStreamSynchronize(c->stream));
@@ -1244,8 +1266,7 @@ int trg_enqueue_steps(trg_ctx* c, int nsteps, double dt_next_checkpoint) {
 	int rc = ensure_dt_hist(c, c->steps + nsteps);
 	if (rc) return rc;
 	for (int s = 0; s < nsteps; ++s) enqueue_full_step(c, dt_next_checkpoint);
-	CUDA_TRY(cudaGetLastError());
-	return TRG_OK;
+	return report_launch_error(c);
 }
 
 void* trg_stream(const trg_ctx* c) { return c ? (void*)c->stream : nullptr; }
@@ -1562,7 +1583,7 @@ int trg_conservation_sums(trg_ctx* c, double* mass, double* energy) {
 	double h[2] = {0, 0};
 	CUDA_TRY(cudaMemcpyAsync(h, c->cons_out, sizeof h, cudaMemcpyDeviceToHost, c->stream));
 	CUDA_TRY(cudaStreamSynchronize(c->stream));
-	CUDA_TRY(cudaGetLastError());
+	if (int rc = report_launch_error(c)) return rc;
 	if (mass) *mass = h[0];
 	if (energy) *energy = h[1];
 	return TRG_OK;
@@ -2039,6 +2060,7 @@ void batch_step(trg_batch* b, double dt_next) {
 	const long long before = v->launches;
 	cudaGraph_t graph = nullptr;
 	bool captured = false;
+	keep_launch_error(v);
 	if (cudaStreamBeginCapture(v->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
 		v->step_capture = true;
 		enqueue_full_step(v, dt_next);
@@ -2048,7 +2070,10 @@ void batch_step(trg_batch* b, double dt_next) {
 	v->use_graphs = use_graphs;
 	if (captured && cudaGraphInstantiate(&g.exec, graph, 0) != cudaSuccess) g.exec = nullptr;
 	if (graph) cudaGraphDestroy(graph);
-	cudaGetLastError();
+	if (cudaGetLastError() != cudaSuccess && g.exec) {  // it lacks a launch, see capture_graph
+		cudaGraphExecDestroy(g.exec);
+		g.exec = nullptr;
+	}
 	g.nodes = v->launches - before;
 	g.q_fresh1 = v->q_fresh;
 	g.colden_valid1 = v->colden_valid;
@@ -2105,9 +2130,7 @@ int trg_batch_learned_start(trg_batch* b, const trg_mlp* m) {
 int trg_batch_enqueue_steps(trg_batch* b, int nsteps, double dt_next_checkpoint) {
 	if (!b || nsteps < 0) return TRG_ERR_ARG;
 	for (int s = 0; s < nsteps; ++s) batch_step(b, dt_next_checkpoint);
-	trg_ctx* c = b->v;
-	CUDA_TRY(cudaGetLastError());
-	return TRG_OK;
+	return report_launch_error(b->v);
 }
 
 int trg_batch_set_conserved(trg_batch* b, int g, const double* U) {
