@@ -95,3 +95,39 @@ def test_refused_launches_of_a_batch_are_reported(gpu, form):
         assert gpu.counts()["refused"], name
         gpu.refuse("")
         b.close()
+
+
+# ------------------------------------------------- shared memory of the chains
+def strip(nx):
+    """2-D, nx shells of at most 5 cells."""
+    tp, ic = workloads.blister((nx, 3, 1), side=0.5 * workloads.PC2CM)
+    return dataclasses.replace(tp, windCellRadius=0, massLossRate=0.0), ic
+
+
+@pytest.mark.parametrize("form", [FP64, FP32])
+@pytest.mark.parametrize("cells, chained", [(57000, True), (60000, False)])
+def test_sweeps_of_very_many_shells_fit_a_cta_or_run_shell_by_shell(gpu, form, cells, chained):
+    tp, ic = known_answers.spitzer_case(cells, 6.0) if form == FP64 else strip(cells)
+    t = torch_b200.Torch(tp, ic, precision=form)
+    t.run_steps(2)
+    names = [l.name for l in gpu.launches()]
+    t.close()
+    assert gpu.counts()["refused"] == 0
+    for sweep in ("rad", "colden"):
+        assert any(f"k_{sweep}_chain" in n for n in names) == chained
+        assert (sum(f"k_{sweep}_shell" in n for n in names) > cells - 20) == (not chained)
+
+
+def test_batch_of_a_long_and_a_wide_grid_fits_a_cta(gpu):
+    """The largest shell and the largest number of shells of different grids,
+    taken together, ask for more than a CTA has; each grid asks for less."""
+    wide = workloads.blister((500, 1000, 1))
+    wide = dataclasses.replace(wide[0], windCellRadius=0, massLossRate=0.0), wide[1]
+    grids = [torch_b200.Torch(*c) for c in (strip(50000), wide)]
+    b = torch_b200.Batch(grids)
+    gpu.reset()
+    b.run_steps(3, grids[0].dt_max)
+    chains = [l for l in gpu.launches() if "k_colden_chain" in l.name]
+    b.close()
+    assert gpu.counts()["refused"] == 0
+    assert chains and all(l.grid == 2 and 48 * 1024 < l.smem <= 227 * 1024 for l in chains)

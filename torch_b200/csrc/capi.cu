@@ -112,7 +112,6 @@ struct trg_ctx {
 	// shell) and dynamic shared memory
 	struct ChainShape {
 		int threads = 0;
-		long long maxshell = 0, nshell = 0;  // of the sweep, or the largest of a batch's
 		size_t smem = 0;
 	} chain_rad, chain_col;
 	// per-grid scalar kernels (dt, time) run on this many threads: 1, or the
@@ -361,8 +360,6 @@ void sweep_out(trg_ctx* c, bool colden) {
 // largest shell, the ring of three shells and the shells' offsets.
 trg_ctx::ChainShape chain_shape(long long maxshell, long long nshell) {
 	trg_ctx::ChainShape sh;
-	sh.maxshell = maxshell;
-	sh.nshell = nshell;
 	sh.threads = 2 * (int)std::min<long long>(CHAIN_GROUP, (maxshell + 31) / 32 * 32);
 	sh.smem = 48 * (size_t)maxshell + sizeof(int) * (size_t)(nshell + 1);
 	return sh;
@@ -888,8 +885,11 @@ int check_device_error(trg_ctx* c) {
 // build, 2.67 against 3.30 in the exact one; 300 x 400: 1.00 against 1.24 and
 // 1.48 against 2.48; 13^3, largest shell 866: 30 against 30 us and 45 against
 // 55), and beyond it for the column densities, whose cells take little
-// arithmetic (400 x 520: 0.61 against 1.74 ms).
+// arithmetic (400 x 520: 0.61 against 1.74 ms); and where the ring and the
+// shells' offsets fit the 227 KB of shared memory that a CTA can have, which a
+// 1-D grid of 58,000 cells exceeds.
 constexpr long long CHAIN_MAX_SHELL_RAD = 1024, CHAIN_MAX_SHELL_COL = 2048;
+constexpr size_t CHAIN_MAX_SMEM = 227 * 1024;
 int build_chain(trg_ctx* c, const std::vector<long long>& off, const int* d_cells, bool rad,
                 const SweepChain** out, trg_ctx::ChainShape* shape) {
 	const long long most = rad ? CHAIN_MAX_SHELL_RAD : CHAIN_MAX_SHELL_COL;
@@ -900,6 +900,8 @@ int build_chain(trg_ctx* c, const std::vector<long long>& off, const int* d_cell
 	std::vector<int> ioff(1, 0);
 	for (long long o : off)
 		if (o > ioff.back()) ioff.push_back((int)o);
+	const trg_ctx::ChainShape sh = chain_shape(maxshell, (long long)ioff.size() - 1);
+	if (sh.smem > CHAIN_MAX_SMEM) return TRG_OK;
 	SweepChain ch;
 	ch.nshell = (int)ioff.size() - 1;
 	ch.n = ioff.back();
@@ -928,7 +930,7 @@ int build_chain(trg_ctx* c, const std::vector<long long>& off, const int* d_cell
 	CUDA_TRY(cudaStreamSynchronize(c->stream));
 	if (h_bad) return TRG_OK;
 	*out = dev;
-	*shape = chain_shape(maxshell, ch.nshell);
+	*shape = sh;
 	return TRG_OK;
 }
 
@@ -2001,16 +2003,18 @@ int trg_batch_create(trg_ctx* const* grids, int G, trg_batch** out) {
 	v->S.sw_rad = v->S.sw_col = nullptr;  // batches read each grid's cells in place
 	v->S.thq = nullptr;
 	v->S.sw_rad_n = v->S.sw_col_n = 0;
-	// sweeps as chains, a cluster per grid, where every grid's are
+	// sweeps as chains, a CTA per grid, where every grid's are: the threads and
+	// the shared memory of the grid that asks for most (each grid lays its own
+	// out), so a batch fits where its grids do
 	auto batch_chain = [&](trg_ctx::ChainShape trg_ctx::*which) {
-		long long maxshell = 0, nshell = 0;
+		trg_ctx::ChainShape most;
 		for (int g = 0; g < G; ++g) {
 			const trg_ctx::ChainShape& sh = grids[g]->*which;
 			if (!sh.threads) return;
-			maxshell = std::max(maxshell, sh.maxshell);
-			nshell = std::max(nshell, sh.nshell);
+			most.threads = std::max(most.threads, sh.threads);
+			most.smem = std::max(most.smem, sh.smem);
 		}
-		v->*which = chain_shape(maxshell, nshell);
+		v->*which = most;
 	};
 	batch_chain(&trg_ctx::chain_rad);
 	batch_chain(&trg_ctx::chain_col);
