@@ -131,3 +131,18 @@ def test_batch_of_a_long_and_a_wide_grid_fits_a_cta(gpu):
     b.close()
     assert gpu.counts()["refused"] == 0
     assert chains and all(l.grid == 2 and 48 * 1024 < l.smem <= 227 * 1024 for l in chains)
+
+
+def test_kernel_attributes_do_not_depend_on_the_grid(gpu):
+    """A kernel's shared-memory limit belongs to the device: set to one grid's
+    need, it would fail another thread's larger grid between setting and launch."""
+    for form in (FP64, FP32):
+        grids = [torch_b200.Torch(*blister(nx, ny), precision=form) for nx, ny in ((300, 400), (20, 33))]
+        for t in grids:
+            t.run_steps(4)
+        batch = [torch_b200.Torch(*blister(nx, ny), precision=form) for nx, ny in ((61, 17), (120, 90))]
+        b = torch_b200.Batch(batch)
+        b.run_steps(4, batch[0].dt_max)
+        b.close()
+    assert any("k_rad_chain" in l.name for l in gpu.launches())
+    assert gpu.most_smem_settings() == 1

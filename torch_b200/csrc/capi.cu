@@ -356,6 +356,7 @@ void sweep_out(trg_ctx* c, bool colden) {
 	if (c->xfn(c->xuser, TRG_EXCHANGE_SWEEP_OUT, c->stream) != 0) c->xfail = true;
 }
 
+constexpr size_t CHAIN_MAX_SMEM = 227 * 1024;
 // The launch shape of a chained sweep: two groups of a thread per cell of the
 // largest shell, the ring of three shells and the shells' offsets.
 trg_ctx::ChainShape chain_shape(long long maxshell, long long nshell) {
@@ -366,7 +367,9 @@ trg_ctx::ChainShape chain_shape(long long maxshell, long long nshell) {
 }
 template <typename... KArgs, typename... Args>
 void launch_chain(trg_ctx* c, const char* name, void (*kernel)(KArgs...), const trg_ctx::ChainShape& sh, Args... args) {
-	cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem);
+	// (the attribute is the kernel's, not the context's: every context sets the
+	// same value, so that none lowers it between another thread's call and launch)
+	cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CHAIN_MAX_SMEM);
 	cudaEvent_t ea = nullptr, eb = nullptr;
 	if (c->profiling) { ea = pool_event(c); eb = pool_event(c); cudaEventRecord(ea, c->stream); }
 	launch_next(c, kernel, (long long)c->nscalar * sh.threads, sh.threads, sh.smem, args...);
@@ -889,7 +892,6 @@ int check_device_error(trg_ctx* c) {
 // shells' offsets fit the 227 KB of shared memory that a CTA can have, which a
 // 1-D grid of 58,000 cells exceeds.
 constexpr long long CHAIN_MAX_SHELL_RAD = 1024, CHAIN_MAX_SHELL_COL = 2048;
-constexpr size_t CHAIN_MAX_SMEM = 227 * 1024;
 int build_chain(trg_ctx* c, const std::vector<long long>& off, const int* d_cells, bool rad,
                 const SweepChain** out, trg_ctx::ChainShape* shape) {
 	const long long most = rad ? CHAIN_MAX_SHELL_RAD : CHAIN_MAX_SHELL_COL;
