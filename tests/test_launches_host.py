@@ -146,3 +146,25 @@ def test_kernel_attributes_do_not_depend_on_the_grid(gpu):
         b.close()
     assert any("k_rad_chain" in l.name for l in gpu.launches())
     assert gpu.most_smem_settings() == 1
+
+
+# ------------------------------------------------------- overlapped launches
+@pytest.mark.parametrize("case", sorted(CASES))
+def test_shell_overlap_switch_covers_every_launch(gpu, monkeypatch, case):
+    """With TRG_SHELL_OVERLAP=0 no kernel may start while the one ahead of it
+    runs; without, the step's kernels may."""
+    make, form = CASES[case]
+    tp, ic = make()
+    for off in (False, True):
+        if off:
+            monkeypatch.setenv("TRG_SHELL_OVERLAP", "0")
+        else:
+            monkeypatch.delenv("TRG_SHELL_OVERLAP", raising=False)
+        gpu.reset()
+        t = torch_b200.Torch(tp, ic, precision=form)
+        t.run_steps(6)
+        if form == FP32:
+            t.autotune()
+        t.close()
+        ahead = [l.name for l in gpu.launches() if l.programmatic]
+        assert not ahead if off else len(ahead) > 6

@@ -102,9 +102,9 @@ struct trg_ctx {
 	long long g_tau_nodes = 0;
 	long long g_colden_nodes = 0, g_rad_nodes[2] = {0, 0};
 	bool use_graphs = true;
-	// shells after the first of a sweep start while the previous one runs
-	// (programmatic dependent launch), and small grids walk all of them in one
-	// launch; TRG_SHELL_OVERLAP=0 launches them one after another
+	// a step's kernels and a sweep's shells after the first start while the one
+	// ahead runs (programmatic dependent launch), and small grids walk all shells
+	// in one launch; TRG_SHELL_OVERLAP=0 launches them one after another
 	bool shell_overlap = shell_overlap_default();
 	// a batch's whole step is being captured (with its side stream's joins)
 	bool step_capture = false;
@@ -657,7 +657,7 @@ void sub_step(trg_ctx* c, double h, bool hasCalculatedHeatFlux, int comp, bool l
 				LAUNCH(KF(k_fb_faces), 148LL * 8 * 128, 128, c->P, c->S);
 			}
 			if (c->profiling) { ea = pool_event(c); eb = pool_event(c); cudaEventRecord(ea, c->stream); }
-			launch_hydro_substep_fp32(c->P, c->S, c->S.U, c->S.U1, h, c->zchunk, c->stream);
+			launch_hydro_substep_fp32(c->P, c->S, c->S.U, c->S.U1, h, c->zchunk, c->stream, c->shell_overlap);
 			if (c->profiling) { cudaEventRecord(eb, c->stream); c->recs.push_back({"k_hydro_stage_fp32", ea, eb}); }
 			c->launches++;
 			// part 2: their FP64 update overwrites the FP32 result
@@ -778,7 +778,7 @@ void enqueue_full_step_fp32(trg_ctx* c, double dt_next) {
 		halo_exchange(c, Uq, true);
 		cudaEvent_t ea = nullptr, eb = nullptr;
 		if (c->profiling) { ea = pool_event(c); eb = pool_event(c); cudaEventRecord(ea, c->stream); }
-		launch_hydro_stage_fp32(st, c->P, c->S, Uq, Ub, Uo, c->zchunk, c->stream);
+		launch_hydro_stage_fp32(st, c->P, c->S, Uq, Ub, Uo, c->zchunk, c->stream, c->shell_overlap);
 		if (c->profiling) { cudaEventRecord(eb, c->stream); c->recs.push_back({"k_hydro_stage_fp32", ea, eb}); }
 		c->launches++;
 	};
@@ -970,6 +970,7 @@ namespace trg {
 const Params& ctx_params(const trg_ctx* c) { return c->P; }
 State ctx_state(const trg_ctx* c) { return c->S; }
 int ctx_device(const trg_ctx* c) { return c->raw.device; }
+bool ctx_overlap(const trg_ctx* c) { return c->shell_overlap; }
 // Planes per CTA of the FP32 hydro pass on this grid.  A CTA's time is its
 // planes and about 3.5 more (the planes before its first are loaded and one of
 // them computed), and two CTAs fit on an SM: the depth is the one whose CTAs,
@@ -1730,8 +1731,8 @@ int trg_autotune(trg_ctx* c, int* zchunk_out, double* ms_out) {
 	CUDA_TRY(cudaEventCreate(&e0));
 	CUDA_TRY(cudaEventCreate(&e1));
 	auto trial = [&](int zc) {
-		if (c->fp32) launch_hydro_stage_fp32(1, c->P, c->S, c->U32, c->U32, c->U32s, zc, c->stream);
-		else launch_hydro_substep_fp32(c->P, c->S, c->S.U, c->S.U1, 0.5, zc, c->stream);
+		if (c->fp32) launch_hydro_stage_fp32(1, c->P, c->S, c->U32, c->U32, c->U32s, zc, c->stream, c->shell_overlap);
+		else launch_hydro_substep_fp32(c->P, c->S, c->S.U, c->S.U1, 0.5, zc, c->stream, c->shell_overlap);
 	};
 	// Launches before the timed ones bring the SM clock up from idle (the
 	// first candidates would otherwise be timed at a lower clock than the

@@ -1211,9 +1211,11 @@ static bool state_tensor_map(const Params& P, const double* U, CUtensorMap* m) {
 	           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// overlap: the launch may start while the kernel ahead of it in the stream runs
+// (grid_begin waits for it).
 template <int STAGE, typename TS, int LIM, int RS>
 static void launch_one(const Params& P, const State& S, const TS* Uq, const TS* Ubase, TS* Uout, double hfac,
-                       int zchunk, cudaStream_t stream) {
+                       int zchunk, cudaStream_t stream, bool overlap) {
 	size_t smem = hydro_stage_fp32_smem();
 	int zc = P.nd > 2 ? zchunk : 1;
 	dim3 grid((P.nx + BX - 1) / BX, (P.ny + BY - 1) / BY, P.nd > 2 ? (P.nz + zc - 1) / zc : 1);
@@ -1233,31 +1235,31 @@ static void launch_one(const Params& P, const State& S, const TS* Uq, const TS* 
 	attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
 	attr[0].val.programmaticStreamSerializationAllowed = 1;
 	cfg.attrs = attr;
-	cfg.numAttrs = 1;
+	cfg.numAttrs = overlap ? 1 : 0;
 	cudaLaunchKernelEx(&cfg, k_hydro_stage_fp32<STAGE, TS, LIM, RS>, P, S, Uq, Ubase, Uout, hfac, zc, tmap, use_tma);
 }
 
 // the reference's configured and default pair (albada, RotatedHLLC) is compiled
 // with both fixed; any other pair takes the run-time switches
 void launch_hydro_stage_fp32(int stage, const Params& P, const State& S, const float* Uq, const float* Ubase,
-                             float* Uout, int zchunk, cudaStream_t stream) {
+                             float* Uout, int zchunk, cudaStream_t stream, bool overlap) {
 	bool fast = P.limiter == 6 && P.riemann == RS_ROTATED;
 	if (stage == 1) {
-		if (fast) launch_one<1, float, 6, RS_ROTATED>(P, S, Uq, Ubase, Uout, 0.5, zchunk, stream);
-		else launch_one<1, float, -1, -1>(P, S, Uq, Ubase, Uout, 0.5, zchunk, stream);
+		if (fast) launch_one<1, float, 6, RS_ROTATED>(P, S, Uq, Ubase, Uout, 0.5, zchunk, stream, overlap);
+		else launch_one<1, float, -1, -1>(P, S, Uq, Ubase, Uout, 0.5, zchunk, stream, overlap);
 	} else {
-		if (fast) launch_one<2, float, 6, RS_ROTATED>(P, S, Uq, Ubase, Uout, 1.0, zchunk, stream);
-		else launch_one<2, float, -1, -1>(P, S, Uq, Ubase, Uout, 1.0, zchunk, stream);
+		if (fast) launch_one<2, float, 6, RS_ROTATED>(P, S, Uq, Ubase, Uout, 1.0, zchunk, stream, overlap);
+		else launch_one<2, float, -1, -1>(P, S, Uq, Ubase, Uout, 1.0, zchunk, stream, overlap);
 	}
 }
 
 // Hydro sub-step of the operator split in the FP32 form, on the FP64 state:
 // Uout = fix(U + h dt L(fixPrimitives(Q(U)))).
 void launch_hydro_substep_fp32(const Params& P, const State& S, const double* U, double* Uout, double h, int zchunk,
-                               cudaStream_t stream) {
+                               cudaStream_t stream, bool overlap) {
 	bool fast = P.limiter == 6 && P.riemann == RS_ROTATED;
-	if (fast) launch_one<1, double, 6, RS_ROTATED>(P, S, U, U, Uout, h, zchunk, stream);
-	else launch_one<1, double, -1, -1>(P, S, U, U, Uout, h, zchunk, stream);
+	if (fast) launch_one<1, double, 6, RS_ROTATED>(P, S, U, U, Uout, h, zchunk, stream, overlap);
+	else launch_one<1, double, -1, -1>(P, S, U, U, Uout, h, zchunk, stream, overlap);
 }
 
 // x-slab decomposition: the two x layers next to each PARTITION face of a

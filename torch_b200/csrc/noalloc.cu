@@ -128,8 +128,8 @@ extern "C" int trg_hydro_step_fp32_noalloc(trg_ctx* c, const double* U_in, doubl
 	k_noalloc_begin<<<1, 1, 0, st>>>(scal, err, dt, P.dt_max);
 	k_f64_to_f32<<<(unsigned)((7 * N + 255) / 256), 256, 0, st>>>(P, U_in, U0);
 	int zchunk = ctx_fp32_zchunk(c);
-	launch_hydro_stage_fp32(1, P, S, U0, U0, Us, zchunk, st);
-	launch_hydro_stage_fp32(2, P, S, Us, U0, U0, zchunk, st);
+	launch_hydro_stage_fp32(1, P, S, U0, U0, Us, zchunk, st, ctx_overlap(c));
+	launch_hydro_stage_fp32(2, P, S, Us, U0, U0, zchunk, st, ctx_overlap(c));
 	k_f32_to_f64<<<(unsigned)((7 * N + 255) / 256), 256, 0, st>>>(P, U0, U_out);
 	// header bytes 16..67: the CFL minimum (scal[2], bits of a positive double)
 	// up to the error word (float 16 = byte 64), read back in one copy

@@ -66,10 +66,10 @@ TRG_FP64_KERNELS
 }
 // FP32 form of the hydro pass (kernels_fp32.cu)
 void launch_hydro_stage_fp32(int stage, const Params& P, const State& S, const float* Uq, const float* Ubase,
-                             float* Uout, int zchunk, cudaStream_t stream);
+                             float* Uout, int zchunk, cudaStream_t stream, bool overlap);
 size_t hydro_stage_fp32_smem();
 void launch_hydro_substep_fp32(const Params& P, const State& S, const double* U, double* Uout, double h, int zchunk,
-                               cudaStream_t stream);
+                               cudaStream_t stream, bool overlap);
 __global__ void k_f64_to_f32(Params P, const double* a, float* b);
 // x-slab decomposition: pack the layers next to the partition faces into dst
 // (kernels_fp32.cu); src is [7][N] doubles, or floats when f32
