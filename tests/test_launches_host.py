@@ -1,6 +1,7 @@
 """What the library launches and reports, on a CUDA runtime that runs nothing
 (fake_gpu)."""
 import dataclasses
+import struct
 
 import numpy as np
 import pytest
@@ -168,3 +169,21 @@ def test_shell_overlap_switch_covers_every_launch(gpu, monkeypatch, case):
         t.close()
         ahead = [l.name for l in gpu.launches() if l.programmatic]
         assert not ahead if off else len(ahead) > 6
+
+
+# ------------------------------------------------------ restored checkpoints
+@pytest.mark.parametrize("case, kept", [("hii_fp32", False), ("blister_fp64", False), ("sedov_fp32", True)])
+def test_restored_time_step_minima_do_not_wait_for_a_kernel(gpu, case, kept):
+    """A blob of a build that left the last step's minima in it: they are dt_max
+    once the call has returned, with no kernel run after the copy (the hydro-only
+    FP32 form's are the next step's limit and stay)."""
+    make, form = CASES[case]
+    t = torch_b200.Torch(*make(), precision=form)
+    at = 8 + 2 * 4 + 8 + 4 * 4 + 8 + 4 * 4  # the header's scalars: dt, time, three minima, block count
+    blob = bytearray(t.checkpoint())
+    blob[at:at + 48] = struct.pack("6d", 0.25, 0.5, 1e-9, 2e-9, 3e-9, 7.0)
+    t.restore(bytes(blob))
+    got = struct.unpack("6d", t.checkpoint()[at:at + 48])
+    want = (1e-9, 2e-9, 3e-9) if kept else (t.dt_max,) * 3
+    t.close()
+    assert got == (0.25, 0.5) + want + (0.0,)

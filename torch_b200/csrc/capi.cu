@@ -1461,10 +1461,13 @@ int trg_checkpoint_load(trg_ctx* c, const void* buf, long long bytes) {
 		p += a.second * sizeof(double);
 	}
 	if (c->fp32) CUDA_TRY(cudaMemcpy(c->U32, p, 7 * N * sizeof(float), cudaMemcpyHostToDevice));
-	CUDA_TRY(cudaMemcpy(c->S.scal, h.scal, sizeof(h.scal), cudaMemcpyHostToDevice));
 	// the time-step minima start from dt_max (the hydro-only FP32 form's hold
-	// the next step's limit), whatever an earlier build left in the blob
-	if (!c->fp32) LAUNCH_SCALAR(KF(k_dt_reset), c->P, c->S);
+	// the next step's limit) and the count of blocks from 0, whatever an earlier
+	// build left in the blob; set here, since a kernel on the context's stream
+	// would not wait for the copy
+	if (!c->fp32) std::fill(h.scal + 2, h.scal + 5, c->P.dt_max);
+	h.scal[SCAL_BLOCKS] = 0;
+	CUDA_TRY(cudaMemcpy(c->S.scal, h.scal, sizeof(h.scal), cudaMemcpyHostToDevice));
 	CUDA_TRY(cudaMemset(c->S.UDOT, 0, 7 * N * sizeof(double)));
 	c->q_fresh = h.q_fresh != 0;
 	c->colden_valid = false;

@@ -1991,7 +1991,7 @@ __global__ void k_dt_finalize(Params P, State S, double dt_next, int first_time,
 	b_dt_finalize(P, S, dt_next, first_time, step);
 }
 // The minima from dt_max again, after a reduction whose minima the host read
-// and after a restored checkpoint (single grids).
+// (single grids).
 __global__ void k_dt_reset(Params P, State S) {
 	grid_begin();
 	b_dt_reset(P, S);
