@@ -2005,16 +2005,7 @@ __global__ void k_dt_reset(Params P, State S) {
 // pass lists those cells; their faces are computed in FP64 from the
 // sub-step's primitives before the FP32 pass overwrites Q, and their update
 // (FP64, with Q of the result) follows the FP32 pass, overwriting its values.
-__device__ __forceinline__ long long clamp_nb(const Params& P, const int* ijk, int dim, int off) {
-	int t[3] = {ijk[0], ijk[1], ijk[2]};
-	const int n = ncell(P, dim);
-	int v = (dim == 0 ? t[0] : dim == 1 ? t[1] : t[2]) + off;
-	v = v < 0 ? 0 : (v >= n ? n - 1 : v);
-	if (dim == 0) t[0] = v;
-	else if (dim == 1) t[1] = v;
-	else t[2] = v;
-	return flat_id(P, t[0], t[1], t[2]);
-}
+//
 // The flag of a cell: its pressure and those of its neighbours up to 2 cells
 // away along each axis (indices clamped to the grid) span a ratio above
 // `contrast`.  A CTA owns a 32 x 8 tile of columns and marches along z through

@@ -179,19 +179,6 @@ __device__ __forceinline__ bool is_wind(const Params& P, long long id, const int
 
 // ---------------------------------------------------------------- algebra
 // GridCell.cpp:163-213.
-__device__ __forceinline__ void UfromQ(double* u, const double* q, double gamma, int nd) {
-	double ke = 0;
-	u[DEN] = q[DEN];
-	#pragma unroll
-	for (int dim = 0; dim < 3; ++dim) if (dim < nd) {
-		u[VEL + dim] = q[VEL + dim] * q[DEN];
-		ke += 0.5 * q[DEN] * q[VEL + dim] * q[VEL + dim];
-	}
-	u[PRE] = q[PRE] / (gamma - 1.0) + ke;
-	u[HII] = q[HII] * q[DEN];
-	u[ADV] = q[ADV] * q[DEN];
-}
-
 __device__ __forceinline__ void QfromU(double* q, const double* u, double gamma, int nd) {
 	Recip r;
 	r.set(u[DEN]);
@@ -222,23 +209,6 @@ __device__ __forceinline__ void QfromU(double* q, const double* u, double gamma,
 		q[ADV] = u[ADV] / u[DEN];
 	}
 	q[PRE] = (u[PRE] - ke) * (gamma - 1.0);
-}
-
-__device__ __forceinline__ void FfromQ(double* f, const double* q, double gamma, int nd, int dim) {
-	f[DEN] = q[DEN] * q[VEL + dim];
-	double ke = 0;
-	#pragma unroll
-	for (int id = 0; id < 3; ++id) if (id < nd) {
-		ke += q[VEL + id] * q[VEL + id];
-		int c = (dim + id) % nd;
-		f[VEL + c] = q[DEN] * q[VEL + c] * q[VEL + dim];
-	}
-	ke *= 0.5 * q[DEN];
-	f[VEL + dim] += q[PRE];
-	double g2 = gamma / (gamma - 1.0);
-	f[PRE] = q[VEL + dim] * (g2 * q[PRE] + ke);
-	f[HII] = q[DEN] * q[VEL + dim] * q[HII];
-	f[ADV] = q[DEN] * q[VEL + dim] * q[ADV];
 }
 
 // Fluid::calcTemperature, Fluid.cpp:71-74.
